@@ -17,13 +17,13 @@ CSRC = os.path.join(PKG, "csrc")
 LIBDIR = os.path.join(PKG, "lib")
 LIB = os.path.join(LIBDIR, "libetb200_sampler.so")
 
-SOURCES = ["sampler_kernels.cu", "c_api.cu", "static_scratch.cu"]
+SOURCES = ["sampler_kernels.cu", "fast_path.cu", "c_api.cu", "static_scratch.cu"]
 HEADERS = sorted(f for f in os.listdir(CSRC) if f.endswith(".cuh")) + [
     os.path.join("..", "..", "include", "etb200_sampler.h")]
 
 NVCC_FLAGS = [
     "-std=c++17", "-O3", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
-    "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden", "--shared",
+    "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden", "--shared", "--threads", "0",
 ]
 
 

@@ -43,18 +43,17 @@ struct etb200_sampler {
   uint64_t launches = 0;
   int blocks_per_sm[3] = {0, 0, 0};  // occupancy of the sampling kernel per dtype, queried once
   ExpTable table;
-  // Rows that the cluster kernel leaves undecided: [0], [1] are the counters of alternating
-  // launches (each launch clears the other one), [2...] the row numbers.
+  // Rows that the fast kernels hand on: [0], [1] are the counters of alternating calls (each
+  // call clears the other one), [2...] the row numbers; and what is known about each row.
   int* d_retry = nullptr;
+  RowHead* d_heads = nullptr;
   int64_t retry_cap = 0;
-  void* cluster_scratch = nullptr;  // per-row record lists of the cluster kernel, one batch of rows
-  size_t cluster_scratch_bytes = 0;
+  void* fast_scratch = nullptr;  // unit records of the sweep
+  size_t fast_scratch_bytes = 0;
   unsigned retry_parity = 0;
   unsigned long long wait_ns = 1000000000ull;  // limit of the in-kernel wait for the other ranks
-  // 0: automatic; 1: the one-block-per-row kernel; 2: the cluster-per-row kernels where they
-  // apply; 3: the one-block-per-row kernel with the estimate-guided sum for 16-bit logits
+  // 0: automatic; 1: the one-block-per-row kernel; 2, 3: the fast kernels wherever they apply
   int kernel_choice = 0;
-  int guided_blocks_per_sm[2] = {0, 0};
 };
 
 namespace {
@@ -181,42 +180,47 @@ int grid_blocks(etb200_sampler* h, int dtype, int64_t rows) {
   return (int)(rows < resident ? rows : resident);
 }
 
-etb200_error_t ensure_retry_list(etb200_sampler* h, int64_t rows) {
-  if (rows <= h->retry_cap) return ETB200_OK;
-  if (h->d_retry) {
-    ETB_CUDA(cudaDeviceSynchronize());
-    ETB_CUDA(cudaFree(h->d_retry));
-    h->d_retry = nullptr;
-    h->retry_cap = 0;
+// Retry list, row heads and unit records for a call on `rows` rows.
+etb200_error_t ensure_fast(etb200_sampler* h, int64_t rows) {
+  if (rows > h->retry_cap) {
+    if (h->d_retry) {
+      ETB_CUDA(cudaDeviceSynchronize());
+      ETB_CUDA(cudaFree(h->d_retry));
+      ETB_CUDA(cudaFree(h->d_heads));
+      h->d_retry = nullptr;
+      h->d_heads = nullptr;
+      h->retry_cap = 0;
+    }
+    const size_t bytes = sizeof(int) * (size_t)(rows + 2);
+    cudaError_t e = cudaMalloc(&h->d_retry, bytes);
+    if (e == cudaSuccess) e = cudaMalloc(&h->d_heads, sizeof(RowHead) * (size_t)rows);
+    if (e != cudaSuccess)
+      return fail(ETB200_MEMORY_ALLOCATION_FAILED, "cudaMalloc of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
+    ETB_CUDA(cudaMemset(h->d_retry, 0, 2 * sizeof(int)));
+    h->retry_cap = rows;
   }
-  const size_t bytes = sizeof(int) * (size_t)(rows + 2);
-  cudaError_t e = cudaMalloc(&h->d_retry, bytes);
-  if (e != cudaSuccess)
-    return fail(ETB200_MEMORY_ALLOCATION_FAILED, "cudaMalloc of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
-  ETB_CUDA(cudaMemset(h->d_retry, 0, 2 * sizeof(int)));
-  h->retry_cap = rows;
+  const size_t need = fast_rows_scratch_bytes(h->vocab, rows);
+  if (need > h->fast_scratch_bytes) {
+    if (h->fast_scratch) {
+      ETB_CUDA(cudaDeviceSynchronize());
+      ETB_CUDA(cudaFree(h->fast_scratch));
+      h->fast_scratch = nullptr;
+      h->fast_scratch_bytes = 0;
+    }
+    cudaError_t e = cudaMalloc(&h->fast_scratch, need);
+    if (e != cudaSuccess)
+      return fail(ETB200_MEMORY_ALLOCATION_FAILED, "cudaMalloc of %zu scratch bytes failed: %s", need,
+                  cudaGetErrorString(e));
+    h->fast_scratch_bytes = need;
+  }
   return ETB200_OK;
 }
 
-// Rows per launch of the cluster kernel pair: bounds the record scratch (about 110 KB per row
-// at a 128k vocabulary).
-constexpr int64_t kClusterBatchRows = 1024;
-
-etb200_error_t ensure_cluster_scratch(etb200_sampler* h, int64_t batch_rows) {
-  const size_t need = topp_cluster_scratch_bytes(h->vocab, batch_rows);
-  if (need <= h->cluster_scratch_bytes) return ETB200_OK;
-  if (h->cluster_scratch) {
-    ETB_CUDA(cudaDeviceSynchronize());
-    ETB_CUDA(cudaFree(h->cluster_scratch));
-    h->cluster_scratch = nullptr;
-    h->cluster_scratch_bytes = 0;
-  }
-  cudaError_t e = cudaMalloc(&h->cluster_scratch, need);
-  if (e != cudaSuccess)
-    return fail(ETB200_MEMORY_ALLOCATION_FAILED, "cudaMalloc of %zu scratch bytes failed: %s", need,
-                cudaGetErrorString(e));
-  h->cluster_scratch_bytes = need;
-  return ETB200_OK;
+// The counter of this call's retry list and the one to clear for the next call.
+void next_retry_counters(etb200_sampler* h, int** count, int** count_next) {
+  *count = h->d_retry + (h->retry_parity & 1u);
+  *count_next = h->d_retry + ((h->retry_parity + 1u) & 1u);
+  h->retry_parity += 1u;
 }
 
 etb200_error_t ensure_scratch(etb200_sampler* h, int blocks) {
@@ -268,50 +272,25 @@ etb200_error_t sample_rows_device(
     etb200_error_t err = ensure_scratch(h, blocks);
     if (err != ETB200_OK) return err;
   }
-  // Automatic choice, from measurements on B200: the cluster pair is the quickest way to one
-  // token from one long row (batch-1 decode); from a handful of rows on, one block per row
-  // keeps more rows in flight and wins.
-  const bool cluster_ok = topp_cluster_supported(dtype, logits, rows, h->vocab, row_stride, h->inv_temperature,
-                                                 h->topp, topk);
-  const bool want_cluster =
-      cluster_ok && (h->kernel_choice == 2 || (h->kernel_choice == 0 && rows == 1 && h->vocab >= 65536));
-  const bool want_guided = !want_cluster && h->kernel_choice == 3 && guided_supported(dtype);
-  if (want_cluster || want_guided) {
-    // Two launches: the fast kernel(s) take every row; the rows they leave undecided (rare) are
-    // then sampled by the plain one-block-per-row kernel, which also carries the arrival
-    // barrier of the multi-GPU forms.
-    etb200_error_t err = ensure_retry_list(h, rows);
+  if (h->kernel_choice != 1 && fast_rows_supported(dtype, rows, h->vocab, h->inv_temperature)) {
+    // The fast kernels take every row; the rows they hand on (long nuclei, and the rare row they
+    // cannot decide) are then sampled by the one-block-per-row kernel, which also carries the
+    // arrival barrier of the multi-GPU forms.
+    etb200_error_t err = ensure_fast(h, rows);
     if (err != ETB200_OK) return err;
-    int* count = h->d_retry + (h->retry_parity & 1u);
-    int* count_next = h->d_retry + ((h->retry_parity + 1u) & 1u);
-    h->retry_parity += 1u;
+    int *count, *count_next;
+    next_retry_counters(h, &count, &count_next);
     PeerOut no_barrier = peers;
     no_barrier.epoch = 0ull;
-    if (want_cluster) {
-      const int64_t batch = rows < kClusterBatchRows ? rows : kClusterBatchRows;
-      err = ensure_cluster_scratch(h, batch);
-      if (err != ETB200_OK) return err;
-      ETB_CUDA(launch_topp_cluster(logits, rows, h->vocab, row_stride, h->inv_temperature, h->topp, rng_states,
-                                   out_ids, no_barrier, h->table, h->cluster_scratch, batch, h->d_retry + 2,
-                                   count, count_next, stream));
-      h->launches += 2 * (uint64_t)((rows + batch - 1) / batch);
-    } else {
-      const int slot = dtype == kDtypeHalf ? 0 : 1;
-      if (h->guided_blocks_per_sm[slot] == 0) h->guided_blocks_per_sm[slot] = guided_kernel_max_blocks_per_sm(dtype);
-      const int64_t resident = (int64_t)h->sm_count * h->guided_blocks_per_sm[slot];
-      const int gblocks = (int)(rows < resident ? rows : resident);
-      if (gblocks > blocks) {
-        err = ensure_scratch(h, gblocks);
-        if (err != ETB200_OK) return err;
-      }
-      ETB_CUDA(launch_sample_rows_guided(dtype, logits, rows, h->vocab, row_stride, h->inv_temperature, h->topp,
-                                         topk, rng_states, out_ids, no_barrier, h->scratch, gblocks, h->table,
-                                         h->d_status, h->d_retry + 2, count, count_next, stream));
-      h->launches += 1;
-    }
-    ETB_CUDA(launch_sample_rows(
-        dtype, logits, rows, h->vocab, row_stride, h->inv_temperature, h->topp, topk, rng_states,
-        out_ids, peers, h->scratch, blocks, h->table, h->d_status, stream, h->d_retry + 2, count));
+    unsigned long long launched = 0;
+    ETB_CUDA(launch_fast_rows(dtype, logits, rows, h->vocab, row_stride, h->inv_temperature, h->topp, topk,
+                              RowSettings{nullptr, nullptr, nullptr, 1.0f}, rng_states, out_ids, no_barrier, h->table,
+                              h->fast_scratch, h->d_heads, h->d_retry + 2, count, count_next, h->sm_count, stream,
+                              &launched));
+    h->launches += launched;
+    ETB_CUDA(launch_sample_rows(dtype, logits, rows, h->vocab, row_stride, h->inv_temperature, h->topp, topk,
+                                rng_states, out_ids, peers, h->scratch, blocks, h->table, h->d_status, stream,
+                                RowPass{h->d_retry + 2, count, h->d_heads}));
     h->launches += 1;
     return ETB200_OK;
   }
@@ -363,7 +342,8 @@ etb200_error_t etb200_sampler_destroy(etb200_sampler_t* h) {
   cudaFree(h->d_status);
   cudaFree(h->scratch);
   cudaFree(h->d_retry);
-  cudaFree(h->cluster_scratch);
+  cudaFree(h->d_heads);
+  cudaFree(h->fast_scratch);
   cudaFree(h->d_stage);
   cudaFree(h->d_stage_states);
   cudaFree(h->d_stage_ids);
@@ -503,10 +483,29 @@ etb200_error_t etb200_sampler_sample_rows_ex(
   ed.bias = opt->edit_bias_device;
   ed.n_shared = opt->n_edits;
   const int topk = (h->topk > 0 && h->topk < h->vocab) ? h->topk : 0;
+  const cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (opt->n_edits > 0) {
+    ETB_CUDA(launch_row_edits(dtype, logits_device, rows, h->vocab, row_stride_elems, ed, st));
+    h->launches += 1;
+  }
+  RowPass pass{nullptr, nullptr, nullptr};
+  const float inv_t = h->inv_temperature == 0.0f && opt->temperature_device != nullptr ? 1.0f : h->inv_temperature;
+  if (false && h->kernel_choice != 1 && opt->scale == 1.0f && fast_rows_supported(dtype, rows, h->vocab, inv_t)) {
+    err = ensure_fast(h, rows);
+    if (err != ETB200_OK) return err;
+    int *count, *count_next;
+    next_retry_counters(h, &count, &count_next);
+    unsigned long long launched = 0;
+    ETB_CUDA(launch_fast_rows(dtype, logits_device, rows, h->vocab, row_stride_elems, h->inv_temperature, h->topp, topk,
+                              rs, states, out_ids_device, PeerOut{}, h->table, h->fast_scratch, h->d_heads,
+                              h->d_retry + 2, count, count_next, h->sm_count, st, &launched));
+    h->launches += launched;
+    pass = RowPass{h->d_retry + 2, count, h->d_heads};
+  }
   ETB_CUDA(launch_sample_rows_ext(dtype, logits_device, rows, h->vocab, row_stride_elems, h->inv_temperature,
-                                  h->topp, topk, rs, ed, states, out_ids_device, h->scratch, blocks, h->table,
-                                  h->d_status, static_cast<cudaStream_t>(stream)));
-  h->launches += opt->n_edits > 0 ? 2 : 1;
+                                  h->topp, topk, rs, states, out_ids_device, h->scratch, blocks, h->table,
+                                  h->d_status, st, pass));
+  h->launches += 1;
   return ETB200_OK;
 }
 

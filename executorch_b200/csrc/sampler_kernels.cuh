@@ -67,52 +67,57 @@ int sample_kernel_max_blocks_per_sm(int dtype);
 
 int sampler_threads();
 
+// What the fast path (launch_fast_rows) knows about a row that it hands on.
+struct alignas(16) RowHead {
+  float mx;       // largest scaled logit, as the reference has it
+  float raw_max;  // largest logit
+  float sum;      // exact softmax sum, when known
+  int state;      // kRow...
+};
+constexpr int kRowUnknown = 0;  // nothing is known
+constexpr int kRowSum = 1;      // mx, raw_max and sum are exact
+constexpr int kRowLong = 2;     // the same, and the nucleus is long
+
+// A pass over some of a batch's rows: the *row_count rows named in row_list, with what is known
+// about each row r in heads[r]. All device pointers; null row_list means every row.
+struct RowPass {
+  const int* row_list;
+  const int* row_count;
+  const RowHead* heads;
+};
+
 // temperature != 0: top-k (0 < topk < vocab), else multinomial (topp outside (0,1)) or top-p
 // sampling of every row. rng_states[r] is advanced once per row; out_ids[r] receives the
-// token. Top-k and top-p need `scratch` (sampler_scratch_bytes). With row_list, only the
-// *row_count rows it names are sampled (both are device pointers).
+// token. Top-k and top-p need `scratch` (sampler_scratch_bytes).
 cudaError_t launch_sample_rows(
     int dtype, const void* logits, int64_t rows, int vocab, int64_t row_stride, float inv_t,
     float topp, int topk, unsigned long long* rng_states, int64_t* out_ids, const PeerOut& peers,
     void* scratch, int blocks, const ExpTable& table, int* status, cudaStream_t stream,
-    const int* row_list = nullptr, const int* row_count = nullptr);
+    const RowPass& pass = RowPass{nullptr, nullptr, nullptr});
 
-// launch_sample_rows for 16-bit logits with the estimate-guided exact sum (the default path):
-// every row is sampled unless the kernel cannot decide it, in which case the row -- rng state
-// and output untouched -- is appended to retry_rows (count in *retry_count, which must be zero
-// at launch) and the caller runs launch_sample_rows with that list on the same stream.
-bool guided_supported(int dtype);
-int guided_kernel_max_blocks_per_sm(int dtype);
-cudaError_t launch_sample_rows_guided(
-    int dtype, const void* logits, int64_t rows, int vocab, int64_t row_stride, float inv_t,
-    float topp, int topk, unsigned long long* rng_states, int64_t* out_ids, const PeerOut& peers,
-    void* scratch, int blocks, const ExpTable& table, int* status, int* retry_rows, int* retry_count,
-    int* retry_count_next, cudaStream_t stream);
+// The edits, applied to the logits in place (one thread per edit).
+cudaError_t launch_row_edits(int dtype, void* logits, int64_t rows, int vocab, int64_t row_stride,
+                             const RowEdits& edits, cudaStream_t stream);
 
-// Top-p sampling of bf16 rows with one thread-block cluster per row (an alternative
-// decomposition, selectable per handle): per batch of at most batch_rows rows, one kernel that turns every row into a short list of
-// records in `scratch` (topp_cluster_scratch_bytes) and one that replays them and draws the
-// token. Rows that cannot be decided this way are appended to retry_rows (their count in
-// *retry_count) with their rng state and output untouched; the caller then runs
-// launch_sample_rows with that list on the same stream. *retry_count must be zero when the
-// first kernel starts; *retry_count_next is cleared for the call after this one.
-constexpr int kClusterMinVocab = 256;
-bool topp_cluster_supported(int dtype, const void* logits, int64_t rows, int vocab, int64_t row_stride,
-                            float inv_t, float topp, int topk);
-size_t topp_cluster_scratch_bytes(int vocab, int64_t batch_rows);
-cudaError_t launch_topp_cluster(
-    const void* logits, int64_t rows, int vocab, int64_t row_stride, float inv_t, float topp,
-    unsigned long long* rng_states, int64_t* out_ids, const PeerOut& peers, const ExpTable& table,
-    void* scratch, int64_t batch_rows, int* retry_rows, int* retry_count, int* retry_count_next,
-    cudaStream_t stream);
-
-// The extended form of launch_sample_rows: first the edits are applied to the logits in
-// place (one thread per edit), then every row is sampled with its own settings; a row whose
-// temperature is 0 takes the argmax. `logits` is written only at the edited positions.
+// launch_sample_rows with every row's own settings; a row whose temperature is 0 takes the argmax.
 cudaError_t launch_sample_rows_ext(
-    int dtype, void* logits, int64_t rows, int vocab, int64_t row_stride, float inv_t, float topp,
-    int topk, const RowSettings& settings, const RowEdits& edits, unsigned long long* rng_states,
-    int64_t* out_ids, void* scratch, int blocks, const ExpTable& table, int* status, cudaStream_t stream);
+    int dtype, const void* logits, int64_t rows, int vocab, int64_t row_stride, float inv_t, float topp,
+    int topk, const RowSettings& settings, unsigned long long* rng_states, int64_t* out_ids, void* scratch, int blocks,
+    const ExpTable& table, int* status, cudaStream_t stream, const RowPass& pass = RowPass{nullptr, nullptr, nullptr});
+
+// The fast path (fast_path.cu): a sweep by one thread-block cluster per row and a finishing
+// kernel. It samples every row that it can decide; the others -- RNG state and output untouched --
+// are appended to retry_rows (count in *retry_count, which must be zero at launch), with
+// what is known about them in heads, and the caller runs launch_sample_rows[_ext] over that list
+// on the same stream. *retry_count_next is cleared for the call after this one. *launches is
+// increased by the number of kernels launched.
+bool fast_rows_supported(int dtype, int64_t rows, int vocab, float inv_t);
+size_t fast_rows_scratch_bytes(int vocab, int64_t rows);
+cudaError_t launch_fast_rows(
+    int dtype, const void* logits, int64_t rows, int vocab, int64_t row_stride, float inv_t, float topp, int topk,
+    const RowSettings& settings, unsigned long long* rng_states, int64_t* out_ids, const PeerOut& peers,
+    const ExpTable& table, void* scratch, RowHead* heads, int* retry_rows, int* retry_count, int* retry_count_next,
+    int sm_count, cudaStream_t stream, unsigned long long* launches);
 
 // temperature == 0: greedy argmax of every row.
 cudaError_t launch_argmax_rows(

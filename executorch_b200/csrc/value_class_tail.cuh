@@ -183,9 +183,7 @@ __device__ VcHit vc_walk(S& sm, const RowMath<T, S>& rm, float sum, float cutoff
     if (pos >= rm.vocab) break;                                     // every token is consumed
     if (vc_prob(rm, sm, (uint32_t)win_hi, sum) < cutoff) break;     // nothing below is a candidate
     if (vc.loaded_hi != win_hi) {
-      ETB_CLOCK_BEGIN();
       const bool counted = vc_histogram(sm, rm, win_hi, pack16);
-      ETB_CLOCK_ADD(11);
       if (tid == 0) vc.loaded_hi = counted ? win_hi : -1;
       if (!counted) {
         out.overflow = true;
@@ -235,7 +233,6 @@ __device__ VcHit vc_walk(S& sm, const RowMath<T, S>& rm, float sum, float cutoff
       if (below) vc.ended = 1;
       if (low_key != 0x7fffffff) atomicMin(&vc.last_key, (unsigned)low_key);
       while (any) {
-        ETB_COUNT(12);
         // every thread: its classes' runs in the binade of the running sum
         SeqSummary s[kVcPer], mine;
         seq_identity(&mine);
@@ -550,9 +547,7 @@ __device__ __forceinline__ int value_class_tail(S& sm, const RowMath<T, S>& rm, 
       vc.n_ck = 0;
     }
     __syncthreads();
-    ETB_STAMP(7);
     const VcHit first = vc_walk(sm, rm, sum, cutoff, topp, key_max, key_min, true, pack16);
-    ETB_STAMP(8);
     if (first.overflow) continue;
     if (first.pos <= 0 && !first.found) return -1;  // no candidate at all
     // last_idx and the sum there (sampler.cpp:147-158); without a hit every candidate is kept
@@ -573,7 +568,6 @@ __device__ __forceinline__ int value_class_tail(S& sm, const RowMath<T, S>& rm, 
     }
     break;
   }
-  ETB_STAMP(9);
   const int token = vc_select(sm, rm, sum, key_max, key_min, pos, pstar);
   return token >= 0 ? token : -2;
 }

@@ -242,18 +242,18 @@ ETB200_EXPORT etb200_error_t etb200_selftest_expf(
 
 /* Which sampling kernel a handle uses for temperature != 0 (a tuning and testing knob; no
  * counterpart in the reference). All choices return the same tokens.
- *   0 (default): automatic -- kernel 2 for a single bf16 row of 65536 logits or more (batch-1
- *      decode, where it is the quickest), kernel 1 otherwise.
- *   1: one thread block per row.
- *   2: a thread-block cluster per row plus a finishing kernel (top-p on bf16 rows whose starts
- *      are 16-byte aligned, 256 <= vocab_size <= 262144, temperature > 0, no top-k); other
- *      cases, and rows it cannot decide, fall to kernel 1.
- *   3: kernel 1 with the exact softmax sum formed from estimate-guided integer increments
- *      (16-bit logits); rows it cannot decide fall to kernel 1. */
+ *   0 (default): automatic -- the fast kernels wherever they apply.
+ *   1: one thread block per row, always.
+ *   2, 3: as 0. The fast kernels are a sweep by a thread-block cluster per row that leaves
+ *      estimate-guided integer increments of the softmax sum, and a finishing kernel that joins
+ *      them to the exact sum and draws the token; they take rows of 256 <= vocab_size <= 262137
+ *      logits of any float type and alignment at a positive temperature. Rows whose nucleus is too
+ *      long for the finishing kernel's lists, and the rare row that it cannot decide, fall to
+ *      kernel 1 in a third launch. */
 ETB200_EXPORT etb200_error_t etb200_sampler_set_kernel_choice(etb200_sampler_t* handle, int32_t choice);
 
 /* Diagnostic (synchronises the device): how many rows of the handle's most recent top-p call
- * the fast kernel left undecided and handed to the plain one-block-per-row kernel. */
+ * the fast kernels handed to the plain one-block-per-row kernel. */
 ETB200_EXPORT etb200_error_t etb200_sampler_last_retry_count(etb200_sampler_t* handle, int32_t* out_count);
 
 /* Number of kernels this library has launched through `handle` so far. */
