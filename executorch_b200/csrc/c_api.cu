@@ -490,7 +490,7 @@ etb200_error_t etb200_sampler_sample_rows_ex(
   }
   RowPass pass{nullptr, nullptr, nullptr};
   const float inv_t = h->inv_temperature == 0.0f && opt->temperature_device != nullptr ? 1.0f : h->inv_temperature;
-  if (false && h->kernel_choice != 1 && opt->scale == 1.0f && fast_rows_supported(dtype, rows, h->vocab, inv_t)) {
+  if (h->kernel_choice != 1 && opt->scale == 1.0f && fast_rows_supported(dtype, rows, h->vocab, inv_t)) {
     err = ensure_fast(h, rows);
     if (err != ETB200_OK) return err;
     int *count, *count_next;

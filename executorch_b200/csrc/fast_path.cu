@@ -53,6 +53,24 @@ cudaError_t launch_sweep_t(const SweepArgs& args, int csize, int sm_count, cudaS
   return cudaLaunchKernelEx(&cfg, row_sweep_kernel<T, kUnitsPerWarp>, args);
 }
 
+template <typename T, bool kMulti>
+cudaError_t launch_finish_t(const FinishArgs& fin, const ExpTable& table, cudaStream_t stream) {
+  static OncePerDevice once;
+  const cudaError_t e = func_attr_once(once, reinterpret_cast<const void*>(row_finish_kernel<T, kMulti>),
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FinishShared));
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)fin.s.rows, 1, 1);
+  cfg.blockDim = dim3(kFinThreads, 1, 1);
+  cfg.dynamicSmemBytes = sizeof(FinishShared);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  programmatic_launch(&attr[0]);
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, row_finish_kernel<T, kMulti>, fin, table);
+}
+
 template <typename T>
 cudaError_t launch_pair_t(SweepArgs args, const FinishArgs& fin, const ExpTable& table, int sm_count,
                           cudaStream_t stream) {
@@ -67,22 +85,11 @@ cudaError_t launch_pair_t(SweepArgs args, const FinishArgs& fin, const ExpTable&
   cudaError_t e = two ? launch_sweep_t<T, 2>(args, csize, sm_count, stream)
                       : launch_sweep_t<T, 4>(args, csize, sm_count, stream);
   if (e != cudaSuccess) return e;
-  static OncePerDevice once;
-  e = func_attr_once(once, reinterpret_cast<const void*>(row_finish_kernel<T>),
-                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FinishShared));
-  if (e != cudaSuccess) return e;
   FinishArgs f = fin;
   f.s = args;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)args.rows, 1, 1);
-  cfg.blockDim = dim3(kFinThreads, 1, 1);
-  cfg.dynamicSmemBytes = sizeof(FinishShared);
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  programmatic_launch(&attr[0]);
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, row_finish_kernel<T>, f, table);
+  const bool multi = args.ext.temperature != nullptr || args.ext.topp != nullptr || args.ext.topk != nullptr ||
+                     (args.topk == 0 && !(args.topp > 0.0f && args.topp < 1.0f));
+  return multi ? launch_finish_t<T, true>(f, table, stream) : launch_finish_t<T, false>(f, table, stream);
 }
 
 }  // namespace

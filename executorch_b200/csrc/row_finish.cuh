@@ -21,11 +21,26 @@ constexpr int kFinThreads = kThreads;   // the tail's helpers are written for kT
 constexpr int kFinEvents = 22;          // event units of a row (2 KB of shared memory each)
 constexpr int kFinTables = 4;           // binades in which an event's terms are summarised
 constexpr int kFinTies = 96;            // exact half-way terms
-constexpr int kFinOdd = 1536;           // corrections that change a parity
-constexpr int kFinGroups = 4096;        // lanes that need another look
-constexpr int kFinCand = 3328;          // candidates
+constexpr int kFinOdd = 1024;           // corrections that change a parity
+constexpr int kFinGroups = 6144;        // lanes that need another look
+constexpr int kFinCand = 3072;          // candidates
 constexpr int kFinFirst = 256;          // lanes whose candidates are listed at once
+constexpr int kFinSlots = 12288;         // 16-bit logits: value classes counted from the row's maximum down
+constexpr int kFinClasses = 4096;        // ... and how many of them may hold anything
+constexpr int kFinTiny = 64;             // logits close to zero, listed one by one
+constexpr int kFinListLanes = 1536;      // up to this many lanes list their candidates one by one
 constexpr int kFinQueue = 64;           // a warp's queue of terms to evaluate
+
+// How an event will probably go: the sum enters it in binade k, the lanes in front of lane l (32: all)
+// add up to `front`, the 16 terms of lane l carry it into binade k2, and the lanes behind l add
+// `behind` there. A half-way term on either side changes the increments by *_d when the significand
+// in front of it (*_at increments in) is odd.
+struct __align__(16) EventPlan {
+  int k, l, front, upto;  // upto: with lane l's own increments in binade k
+  int k2, behind;
+  int front_at, front_d, behind_at, behind_d;
+  int ok, pad;
+};
 
 // The tail's share: candidates by probability.
 constexpr int kTailBins = 1024;      // value bins: exponent and 5 mantissa bits, from the floor up
@@ -37,6 +52,55 @@ struct FinishTail {
   alignas(16) float p[kFinCand + 32];       // sorted
   int idx[kFinCand];
 };
+
+// Its share when the candidates are counted by value class instead of listed.
+struct FinishClasses {
+  uint16_t key[kFinClasses];  // order-preserving keys of the classes that hold candidates, descending
+  uint16_t n[kFinClasses];    // how many
+  float p[kFinClasses];       // their probabilities
+  int ck_kb[kFinClasses / 32 + 1], ck_n[kFinClasses / 32 + 1], ck_pos[kFinClasses / 32 + 1];  // the sum in front of every 32
+  int unit_cnt[kSwMaxUnits];
+};
+
+// Slots of the value classes of one row: bit patterns from the largest logit's down, leaving out the
+// patterns of tiny magnitude (the thousands of exponents around zero that no row fills).
+struct ClassSlots {
+  uint32_t tiny, top;  // magnitudes: of the smallest that has a slot, of the row's largest logit
+  bool negative;       // the largest logit is negative
+  // Slot of a pattern; 0x7fffffff for a tiny one, something >= kFinSlots when it is out of range.
+  __device__ __forceinline__ uint32_t slot(uint32_t pat) const {
+    const uint32_t m = pat & 0x7FFFu;
+    if (m < tiny) return 0x7fffffffu;
+    if (!(pat & 0x8000u)) return top - m;
+    return negative ? m - top : (top >= tiny ? top - tiny + 1u : 0u) + (m - tiny);
+  }
+  __device__ __forceinline__ uint32_t pattern(uint32_t slot) const {
+    if (negative) return 0x8000u | (top + slot);
+    const uint32_t pos = top >= tiny ? top - tiny + 1u : 0u;
+    return slot < pos ? top - slot : 0x8000u | (tiny + (slot - pos));
+  }
+  // first slot behind the tiny magnitudes
+  __device__ __forceinline__ uint32_t behind_tiny() const { return negative ? 0u : (top >= tiny ? top - tiny + 1u : 0u); }
+};
+template <typename T>
+__device__ __forceinline__ ClassSlots class_slots(float raw_max) {
+  ClassSlots c;
+  uint32_t pat;
+  if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+    pat = f32_bits(raw_max) >> 16;
+    c.tiny = (127u - 12u) << 7;  // 2^-12
+  } else {
+    pat = (uint32_t)__half_as_ushort(__float2half_rn(raw_max));
+    c.tiny = (15u - 4u) << 10;  // 2^-4
+  }
+  c.negative = (pat & 0x8000u) != 0u;
+  c.top = pat & 0x7FFFu;
+  if (c.negative && c.top < c.tiny) {  // a tiny negative maximum: slots from the smallest magnitude on
+    c.negative = false;
+    c.top = 0u;
+  }
+  return c;
+}
 
 struct __align__(16) FinishShared {
   static constexpr bool kExt = false;
@@ -58,13 +122,16 @@ struct __align__(16) FinishShared {
   int n_task, n_task2, n_cand, n_tie, n_odd, bad;
   float sum, coin, start_sum, mass;
   int ev_unit[kFinEvents + 1];
-  int run_a0[kFinEvents + 1], run_a1[kFinEvents + 1], run_k[kFinEvents + 1];  // between events; k = 0: only zeros
+  float ev_sum[kFinEvents];  // what each event adds to the sum
+  int4 run[kFinEvents + 1];  // between events: increments (entered even, odd), binade (0: only zeros)
   union alignas(16) {
     struct {
       float pool[kFinEvents][kUnit];       // exact terms of the event units, swizzled (pool_chunk)
       uint16_t group[kFinGroups];          // unit * 32 + lane; those with unsure terms first
-      int tab_k[kFinEvents][kFinTables];             // the binades
-      unsigned tab_tie[kFinEvents][kFinTables];      // lanes with an exact half-way term in that binade
+      EventPlan plan[kFinEvents];
+      float ev_tot[kFinEvents];                      // sums of the events' terms, roughly
+      alignas(16) int tab_k[kFinEvents][kFinTables];             // the binades
+      alignas(16) unsigned tab_tie[kFinEvents][kFinTables];      // lanes with an exact half-way term in that binade
       int tab_inc[kFinEvents][kFinTables][32];       // inclusive sums of the lanes' increments
       signed char tab_d[kFinEvents][kFinTables][32]; // change of a lane's increment when entered odd
       uint32_t tie[kFinTies];                        // padded position | kTieUp
@@ -75,9 +142,16 @@ struct __align__(16) FinishShared {
       uint32_t queue[kWarps][kFinQueue];   // terms to evaluate exactly: padded position | kQ...
     };
     FinishTail t;
+    FinishClasses c;
   } u;
-  Entry cand[kFinCand];
+  union {
+    Entry cand[kFinCand];
+    unsigned hist[kFinSlots / 2];  // 16-bit counters, two per word
+  };
+  int cls_over, cls_m, n_counted, n_tiny;
+  uint16_t tiny_key[kFinTiny];
 };
+static_assert(sizeof(FinishClasses) <= sizeof(float) * kFinEvents * kUnit, "the group list behind the pool stays");
 static_assert(sizeof(FinishShared) <= 115712, "two blocks per SM");
 constexpr uint32_t kTieUp = 1u << 31;
 constexpr uint32_t kQCand = 1u << 31, kQUnsure = 1u << 30, kQPos = (1u << 30) - 1u;
@@ -131,6 +205,38 @@ __device__ __forceinline__ void load_unit_lane(const T* row, int shift, int voca
         x[q * 8 + j] = (i >= 0 && i < vocab) ? to_f32(row[i]) : -INFINITY;
       }
   }
+}
+
+// Eight 16-bit logits as bit patterns, two per word.
+template <typename T>
+__device__ __forceinline__ void load4_patterns(const T* row, int shift, int vocab, int p, uint32_t (&w)[4]) {
+  const int i0 = p - shift;
+  const unsigned short* row16 = reinterpret_cast<const unsigned short*>(row);
+  if (i0 >= 0 && i0 + 8 <= vocab) {
+    const uint4 raw = __ldg(reinterpret_cast<const uint4*>(row16 + i0));
+    w[0] = raw.x;
+    w[1] = raw.y;
+    w[2] = raw.z;
+    w[3] = raw.w;
+  } else {
+    const uint32_t ninf = std::is_same<T, __nv_bfloat16>::value ? 0xFF80u : 0xFC00u;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int i = i0 + 2 * k;
+      const uint32_t lo = i >= 0 && i < vocab ? row16[i] : ninf, hi = i + 1 >= 0 && i + 1 < vocab ? row16[i + 1] : ninf;
+      w[k] = lo | (hi << 16);
+    }
+  }
+}
+// key_of_pattern16 of both halves of a word
+__device__ __forceinline__ uint32_t keys_of_word(uint32_t w) {
+  return w ^ 0x80008000u ^ (((w >> 15) & 0x00010001u) * 0x7FFFu);
+}
+template <typename T>
+__device__ __forceinline__ float value_of_key(uint32_t key) {
+  const uint32_t pat = pattern_of_key16(key);
+  if constexpr (std::is_same<T, __nv_bfloat16>::value) return bits_f32(pat << 16);
+  else return __half2float(__ushort_as_half((unsigned short)pat));
 }
 
 struct FinishArgs {
@@ -221,6 +327,12 @@ __device__ __forceinline__ void finish_event(FinishShared& sm, const T* row, int
     v[4 * q + 2] = f.z;
     v[4 * q + 3] = f.w;
   }
+  float tot = 0.0f;
+#pragma unroll
+  for (int j = 0; j < 16; ++j) tot += v[j];
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, d);
+  if (lane == 0) sm.u.ev_tot[e] = tot;
   const uint32_t info = sm.u.info[u];
   const int klo = unit_binade(info), span = (int)unit_span(info);
   const int nt = span == (int)kUnitSpanOpen ? 0 : (span < kFinTables - 1 ? span + 1 : kFinTables);
@@ -274,29 +386,33 @@ __device__ __forceinline__ float finish_apply_event(FinishShared& sm, int e, flo
   int f = 0;  // lanes in front of f are in s
   while (f < 32) {
     const int k = seq_kb(s), n = seq_n(s);
-    const int tk = lane < kFinTables ? sm.u.tab_k[e][lane] : 0;
-    const unsigned has = __ballot_sync(0xffffffffu, tk == k);
+    const unsigned has = __ballot_sync(0xffffffffu, lane < kFinTables && sm.u.tab_k[e][lane & (kFinTables - 1)] == k);
     if (has == 0u) break;
     const int t = __ffs(has) - 1;
     const int inc = sm.u.tab_inc[e][t][lane];
+    unsigned ties = sm.u.tab_tie[e][t];
     const int base = f > 0 ? __shfl_sync(0xffffffffu, inc, f - 1) : 0;
     int end = n + (inc - base);  // the significand behind this lane (lanes from f on)
-    for (unsigned ties = sm.u.tab_tie[e][t] >> f << f; ties != 0u; ties &= ties - 1u) {
+    for (ties = ties >> f << f; ties != 0u; ties &= ties - 1u) {
       const int l = __ffs(ties) - 1;
       const int in = l > f ? __shfl_sync(0xffffffffu, end, l - 1) : n;
       if ((in & 1) && lane >= l) end += sm.u.tab_d[e][t][l];
     }
     const unsigned out = __ballot_sync(0xffffffffu, lane >= f && end >= kSeqLimit);
     const int l = out != 0u ? __ffs(out) - 1 : 32;
-    const int before = __shfl_sync(0xffffffffu, end, l > 0 ? l - 1 : 0);
-    s = seq_value(k, l > f ? before : n);
-    if (l == 32) return s;
+    if (l < 32) {
+      float4 v[4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const float4 v = pool4[pool_chunk(l * 4 + q)];
-      s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, v.x), v.y), v.z), v.w);
+      for (int q = 0; q < 4; ++q) v[q] = pool4[pool_chunk(l * 4 + q)];
+      const int before = __shfl_sync(0xffffffffu, end, l > 0 ? l - 1 : 0);
+      s = seq_value(k, l > f ? before : n);
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, v[q].x), v[q].y), v[q].z), v[q].w);
+      f = l + 1;
+    } else {
+      return seq_value(k, __shfl_sync(0xffffffffu, end, 31));
     }
-    f = l + 1;
   }
   if (f < 32) {
     // no summary for this binade: the general way for the other lanes
@@ -516,7 +632,422 @@ __device__ __forceinline__ bool finish_tail(FinishShared& sm, float e_floor, flo
   return true;
 }
 
-template <typename T>
+// One walk over the value classes [32 * tile, m), from a sum in front of that tile, until the running
+// float sum exceeds thr (by one warp): classes are runs of equal terms with closed-form summaries
+// (class_math.cuh), composed over 32 of them by a scan. Found: *cls, the copy's position in the sorted
+// list, the position of the class's first copy, and the sum there; else the number of entries and
+// their sum. The first walk records the sum in front of every tile.
+__device__ __forceinline__ bool classes_walk(FinishShared& sm, int m, float thr, int tile, int kb, int n, int pos,
+                                             bool record, int* cls, int* at, int* start, float* cum) {
+  const int lane = threadIdx.x & 31;
+  FinishClasses& c = sm.u.c;
+  for (; 32 * tile < m; ++tile) {
+    if (record && lane == 0) {
+      c.ck_kb[tile] = kb;
+      c.ck_n[tile] = n;
+      c.ck_pos[tile] = pos;
+    }
+    const int k = 32 * tile + lane;
+    const float p = k < m ? c.p[k] : 0.0f;
+    const int all = k < m ? (int)c.n[k] : 0;
+    int cnt = all;
+    for (;;) {
+      SeqSummary s = rep_summary(p, cnt, kb);
+      int ic = cnt;
+      const int limit = thr_limit(thr, kb);
+      const bool two = __any_sync(0xffffffffu, s.a0 != s.a1);
+      if (!two) {
+        // the usual tile: nothing in it reaches the limit, and its total is all that is needed
+        const unsigned tot = __reduce_add_sync(0xffffffffu, (unsigned)s.a0);  // at most 32 * 2^26
+        if ((unsigned)n + tot < (unsigned)limit) {
+          n += (int)tot;
+          pos += __reduce_add_sync(0xffffffffu, cnt);
+          break;
+        }
+      }
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        SeqSummary o;
+        o.a0 = __shfl_up_sync(0xffffffffu, s.a0, d);
+        o.a1 = two ? __shfl_up_sync(0xffffffffu, s.a1, d) : o.a0;
+        const int oc = __shfl_up_sync(0xffffffffu, ic, d);
+        if (lane >= d) {
+          s = seq_compose(o, s);
+          ic += oc;
+        }
+      }
+      const int n_out = seq_apply(n, s);
+      const unsigned b = __ballot_sync(0xffffffffu, cnt > 0 && n_out >= limit);
+      if (b == 0u) {
+        n = __shfl_sync(0xffffffffu, n_out, 31);
+        pos += __shfl_sync(0xffffffffu, ic, 31);
+        break;
+      }
+      const int f = __ffs(b) - 1;
+      const int before = __shfl_sync(0xffffffffu, n_out, f > 0 ? f - 1 : 0);
+      WalkState st;
+      st.kb = kb;
+      st.n = f > 0 ? before : n;
+      bool found = false;
+      float sum = 0.0f;
+      int j = 0;
+      if (lane == f) {
+        // a long run may carry the sum through several binades
+        do {
+          j += class_hit_step(&st, p, cnt - j, thr, &found, &sum);
+        } while (!found && j < cnt && seq_apply(st.n, rep_summary(p, cnt - j, st.kb)) >= thr_limit(thr, st.kb));
+      }
+      kb = __shfl_sync(0xffffffffu, st.kb, f);
+      n = __shfl_sync(0xffffffffu, st.n, f);
+      j = __shfl_sync(0xffffffffu, j, f);
+      pos += __shfl_sync(0xffffffffu, ic - cnt, f) + j;
+      const int used = __shfl_sync(0xffffffffu, all - cnt, f) + j;  // copies of class f so far
+      if (__shfl_sync(0xffffffffu, found ? 1 : 0, f)) {
+        *cls = 32 * tile + f;
+        *at = pos - 1;
+        *start = pos - used;
+        *cum = __shfl_sync(0xffffffffu, sum, f);
+        return true;
+      }
+      if (lane < f) cnt = 0;
+      if (lane == f) cnt -= j;
+    }
+  }
+  *at = pos;
+  *cum = seq_value(kb, n);
+  return false;
+}
+
+// Adds the terms of event e to the exact running sum s, looking for the first position at which it
+// exceeds thr (seqsum_warp). p0: position of the event's first term in the row.
+__device__ __forceinline__ bool finish_search_event(FinishShared& sm, int e, float& s, float thr, int p0, int vocab, int* hit) {
+  const int lane = threadIdx.x & 31;
+  const float4* pool4 = reinterpret_cast<const float4*>(sm.u.pool[e]);
+  float v[kChunk];
+#pragma unroll
+  for (int q = 0; q < kChunk / 4; ++q) {
+    const float4 x = pool4[pool_chunk(lane * 4 + q)];
+    v[4 * q] = x.x;
+    v[4 * q + 1] = x.y;
+    v[4 * q + 2] = x.z;
+    v[4 * q + 3] = x.w;
+  }
+  float at;
+  return seqsum_warp<true>(v, s, thr, p0, vocab, hit, &at);
+}
+
+// The rest of sample_topp on the row's value classes (counted in sm.hist and sm.tiny_key): the classes
+// that hold anything with their probabilities, the two walks, and the token of the wanted rank
+// among those of equal probability, by index, with one more look at the lanes that were counted
+// (sm.u.group). Returns as finish_tail.
+template <typename T, typename Term>
+__device__ __forceinline__ bool finish_classes(FinishShared& sm, const T* row, int shift, int vocab, int n_units, int n_groups,
+                                               const ClassSlots& slots, float e_floor, float sum, float cutoff,
+                                               float topp, bool complete, float coin, Term exact_term, int* token,
+                                               float* mass) {
+  constexpr int kPer = kFinSlots / 2 / kFinThreads;  // words per thread
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  FinishClasses& c = sm.u.c;
+  const int n_tiny = sm.n_tiny;
+  if (sm.cls_over || n_tiny > kFinTiny) return false;
+  if (tid == 0) sm.cls_m = 0x7fffffff;
+  // how many classes, and how many logits the counters add up to (a counter that ran over shows)
+  int have = 0, sum_n = 0;
+  unsigned words[kPer];  // 128-bit reads, in distinct banks for eight neighbouring threads
+#pragma unroll
+  for (int k = 0; k < kPer / 4; ++k) {
+    const uint4 q = reinterpret_cast<const uint4*>(sm.hist)[tid * (kPer / 4) + k];
+    words[4 * k] = q.x;
+    words[4 * k + 1] = q.y;
+    words[4 * k + 2] = q.z;
+    words[4 * k + 3] = q.w;
+  }
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    have += (words[k] & 0xFFFFu ? 1 : 0) + (words[k] >> 16 ? 1 : 0);
+    sum_n += (int)(words[k] & 0xFFFFu) + (int)(words[k] >> 16);
+  }
+  const uint32_t split = slots.behind_tiny();
+  int m, counted;
+  int at0 = finish_scan(sm.redi, have, &m);
+  finish_scan(sm.redf_i, sum_n, &counted);
+  if (counted != sm.n_counted || m + n_tiny > kFinClasses) return false;
+  m += n_tiny;
+#pragma unroll
+  for (int k = 0; k < 2 * kPer; ++k) {
+    const unsigned n = k & 1 ? words[k >> 1] >> 16 : words[k >> 1] & 0xFFFFu;
+    if (n != 0u) {
+      const uint32_t sl = (uint32_t)(tid * 2 * kPer + k);
+      const int o = at0++ + (sl >= split ? n_tiny : 0);
+      c.key[o] = (uint16_t)key_of_pattern16(slots.pattern(sl));
+      c.n[o] = (uint16_t)n;
+      if (sl < split && n_tiny > 0) atomicMax(&sm.tail_pos, o);  // (-1 before)
+    }
+  }
+  __syncthreads();
+  if (tid < n_tiny) {
+    // the tiny ones between the two, largest first
+    const uint16_t mine = sm.tiny_key[tid];
+    int o = sm.tail_pos + 1;
+    for (int k = 0; k < n_tiny; ++k) o += sm.tiny_key[k] > mine || (sm.tiny_key[k] == mine && k < tid) ? 1 : 0;
+    c.key[o] = mine;
+    c.n[o] = 1;
+  }
+  __syncthreads();
+  for (int k = tid; k < m; k += kFinThreads) {
+    const float e = exact_term(value_of_key<T>(c.key[k]));
+    const float p = __fdiv_rn(e, sum);
+    c.p[k] = p;
+    // the crop (sampler.cpp:136-143): nothing below is a candidate; and below the floor not everything
+    // was counted
+    if (p < cutoff || e < e_floor) atomicMin(&sm.cls_m, k);
+  }
+  c.unit_cnt[tid] = 0;
+  __syncthreads();
+  if (sm.cls_m < m) m = sm.cls_m;
+  if (warp == 0) {
+    int cls = 0, at = 0, start = 0, n_tiles = (m + 31) / 32;
+    float cum = 0.0f;
+    const bool found = classes_walk(sm, m, topp, 0, 1, 0, 0, true, &cls, &at, &start, &cum);
+    bool ok = m > 0 && (found || complete);
+    if (found) {
+      n_tiles = cls / 32 + 1;
+    } else if (m > 0) {
+      cls = m - 1;  // the sum never exceeded topp: everything is kept (sampler.cpp:152)
+      start = at - (int)c.n[cls];
+      at -= 1;
+    }
+    const float r = __fmul_rn(coin, cum);  // sampler.cpp:162
+    if (ok && r < cum) {
+      __syncwarp();
+      int t = 0;
+      for (int q = lane; q < n_tiles; q += 32)
+        if (seq_value(c.ck_kb[q], c.ck_n[q]) <= r) t = q;
+      t = __reduce_max_sync(0xffffffffu, t);
+      int cls2 = 0, at2 = 0, start2 = 0;
+      float cum2;
+      if (classes_walk(sm, m, r, t, c.ck_kb[t], c.ck_n[t], c.ck_pos[t], false, &cls2, &at2, &start2, &cum2) && at2 <= at) {
+        cls = cls2;
+        at = at2;
+        start = start2;
+      }
+    }
+    if (lane == 0) {
+      // classes of the same float probability are one group, in index order
+      int g0 = cls, g1 = cls, rank = at - start;
+      if (ok) {
+        const float p = c.p[cls];
+        while (g0 > 0 && c.p[g0 - 1] == p) rank += (int)c.n[--g0];
+        while (g1 + 1 < m && c.p[g1 + 1] == p) ++g1;
+      }
+      sm.tail_last = ok ? (int)c.key[g0] : -1;  // the group's keys
+      sm.tail_bin = ok ? (int)c.key[g1] : -1;
+      sm.tail_cnt = rank;
+      sm.tail_mass = cum;
+    }
+  }
+  __syncthreads();
+  *mass = sm.tail_mass;
+  if (sm.tail_last < 0) return false;
+  const uint32_t g_lo = (uint32_t)sm.tail_bin, span = (uint32_t)(sm.tail_last - sm.tail_bin);
+  const int rank = sm.tail_cnt;
+  for (int h0 = tid; h0 < 2 * n_groups; h0 += 4 * kFinThreads) {
+    uint32_t w[4][4];
+    int unit[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {  // four reads of the row in flight
+      const int h = h0 + q * kFinThreads;
+      unit[q] = -1;
+      if (h < 2 * n_groups) {
+        const int g = sm.u.group[h >> 1];
+        unit[q] = g >> 5;
+        load4_patterns(row, shift, vocab, unit[q] * kUnit + unit_pos(g & 31, h & 1), w[q]);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      if (unit[q] < 0) continue;
+      int n = 0;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const uint32_t key = keys_of_word(w[q][k]);
+        n += ((key & 0xFFFFu) - g_lo <= span ? 1 : 0) + ((key >> 16) - g_lo <= span ? 1 : 0);
+      }
+      if (n > 0) atomicAdd(&c.unit_cnt[unit[q]], n);
+    }
+  }
+  if (tid == 0) sm.tail_pos = -1;
+  __syncthreads();
+  int tot;
+  const int mine = tid < n_units ? c.unit_cnt[tid] : 0;
+  const int pre = finish_scan(sm.redf_i, mine, &tot);
+  if (rank >= pre && rank < pre + mine) {
+    sm.tail_bin = tid;
+    sm.tail_cnt = rank - pre;
+    sm.tail_pos = 0;
+  }
+  __syncthreads();
+  if (sm.tail_pos < 0) return false;
+  if (warp == 0) {
+    const int u = sm.tail_bin;
+    int left = sm.tail_cnt;
+    int found = -1;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      uint32_t w[4];
+      load4_patterns(row, shift, vocab, u * kUnit + unit_pos(lane, q), w);
+      unsigned in = 0u;  // this lane's members among its eight logits
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const uint32_t key = keys_of_word(w[k]);
+        in |= ((key & 0xFFFFu) - g_lo <= span ? 1u : 0u) << (2 * k);
+        in |= ((key >> 16) - g_lo <= span ? 1u : 0u) << (2 * k + 1);
+      }
+      const int n = __popc(in);
+      int inc = n;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int o = __shfl_up_sync(0xffffffffu, inc, d);
+        if (lane >= d) inc += o;
+      }
+      if (left >= inc - n && left < inc) {
+        for (int k = left - (inc - n); k > 0; --k) in &= in - 1u;
+        found = u * kUnit + unit_pos(lane, q) + __ffs(in) - 1 - shift;
+      }
+      left -= __shfl_sync(0xffffffffu, inc, 31);
+    }
+    found = __reduce_max_sync(0xffffffffu, found);
+    if (lane == 0) sm.tail_pos = found;
+  }
+  __syncthreads();
+  *token = sm.tail_pos;
+  return true;
+}
+
+// Lane e: the plan of event e, from the sum in front of it as the runs and events in front of it
+// estimate it (good to a few hundred units of the last place; a lane's increments are thousands).
+__device__ __forceinline__ void plan_event(FinishShared& sm, int e, float in) {
+  EventPlan p = {};
+  const int k = seq_kb(in), n = seq_n(in);
+  const int4 tk = *reinterpret_cast<const int4*>(sm.u.tab_k[e]);
+  auto table = [&](int b) { return tk.x == b ? 0 : (tk.y == b ? 1 : (tk.z == b ? 2 : (tk.w == b ? 3 : -1))); };
+  const int t = table(k);
+  if (t >= 0) {
+    const int* inc = sm.u.tab_inc[e][t];
+    int l = 0;
+#pragma unroll
+    for (int step = 16; step > 0; step >>= 1)
+      if (n + inc[l + step - 1] < kSeqLimit) l += step;
+    if (l == 31 && n + inc[31] < kSeqLimit) l = 32;
+    p.k = k;
+    p.l = l;
+    p.front = l > 0 ? inc[l - 1] : 0;
+    p.ok = 1;
+    auto half_way = [&](unsigned ties, const int* a, int tt, int base, int* at, int* d) {
+      if (__popc(ties) > 1) p.ok = 0;
+      if (ties != 0u) {
+        const int q = __ffs(ties) - 1;
+        *at = (q > 0 ? a[q - 1] : 0) - base;
+        *d = sm.u.tab_d[e][tt][q];
+      }
+    };
+    half_way(sm.u.tab_tie[e][t] & (l < 32 ? (1u << l) - 1u : 0xFFFFFFFFu), inc, t, 0, &p.front_at, &p.front_d);
+    if (l < 32) {
+      p.upto = inc[l];
+      const long long after = (long long)n + inc[l];  // in units of binade k
+      p.k2 = k + (31 - __clz((int)(after >> 23)));
+      const int t2 = table(p.k2);
+      if (t2 < 0 || p.k2 == k) {
+        p.ok = 0;
+      } else {
+        const int* inc2 = sm.u.tab_inc[e][t2];
+        p.behind = inc2[31] - inc2[l];
+        if ((after >> (p.k2 - k)) + p.behind >= kSeqLimit - 64) p.ok = 0;  // probably leaves that binade, too
+        half_way(sm.u.tab_tie[e][t2] & (l < 31 ? 0xFFFFFFFFu << (l + 1) : 0u), inc2, t2, inc2[l], &p.behind_at,
+                 &p.behind_d);
+      }
+    }
+  }
+  sm.u.plan[e] = p;
+}
+
+// The exact sequential sum of the row from its runs and events, by one warp; with kMulti up to the
+// first position at which it exceeds thr, looked for in the events from unit hit_unit on (*hit >= 0
+// when there is one). False when an assumption of the sweep does not hold.
+//
+// It is one chain of dependent steps over some ten events, so each step is made short: where an event
+// leaves its binade is worked out beforehand from estimates, a lane per event, and what remains in
+// the chain is to check that, an integer addition, 16 float additions, and another integer addition
+// (130 cycles; the general form with its votes and shuffles takes 1200). An event that goes
+// differently takes the general form.
+template <bool kMulti>
+__device__ __forceinline__ bool finish_replay(FinishShared& sm, int n_ev, float thr, int hit_unit, int shift, int vocab,
+                                           float* sum, int* hit) {
+  const int lane = threadIdx.x & 31;
+  {
+    const int4 r4 = lane <= n_ev ? sm.run[lane] : make_int4(0, 0, 0, 0);
+    const float run = r4.z > 0 ? (float)r4.x * bits_f32((uint32_t)(r4.z > 23 ? r4.z - 23 : 0) << 23) : 0.0f;
+    const float tot = lane < n_ev ? (lane == 0 ? sm.start_sum : sm.u.ev_tot[lane]) : 0.0f;
+    float in = run + tot;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const float o = __shfl_up_sync(0xffffffffu, in, d);
+      if (lane >= d) in += o;
+    }
+    const float before = __shfl_up_sync(0xffffffffu, in, 1);
+    if (lane > 0 && lane < n_ev) plan_event(sm, lane, before + run);
+  }
+  __syncwarp();
+  float s = 0.0f;
+#pragma unroll 1
+  for (int e = 0; e <= n_ev; ++e) {
+    const int4 r4 = sm.run[e];
+    int k = seq_kb(s), n = seq_n(s);
+    if (r4.z != 0) {
+      n += (n & 1) ? r4.y : r4.x;  // at most 2^24 + 2^26
+      if (r4.z != k || n >= kSeqLimit) return false;
+      s = seq_value(k, n);
+      if (kMulti && !(s <= thr)) return false;
+    }
+    if (e == n_ev) break;
+    const float before = s;
+    if (kMulti && sm.ev_unit[e] >= hit_unit) {
+      if (finish_search_event(sm, e, s, thr, sm.ev_unit[e] * kUnit - shift, vocab, hit)) break;
+    } else if (e == 0) {
+      s = sm.start_sum;
+    } else {
+      const EventPlan p = sm.u.plan[e];
+      const float4* pool4 = reinterpret_cast<const float4*>(sm.u.pool[e]);
+      float4 v[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) v[q] = pool4[pool_chunk((p.l & 31) * 4 + q)];
+      int in = n + p.front;
+      if ((n + p.front_at) & 1) in += p.front_d;
+      bool good = p.ok != 0 && p.k == k && in < kSeqLimit;
+      float r = seq_value(k, in);
+      if (p.l < 32) {
+        good = good && n + p.upto >= kSeqLimit + 2;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          r = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(r, v[q].x), v[q].y), v[q].z), v[q].w);
+        const int n2 = seq_n(r);
+        int out = n2 + p.behind;
+        if ((n2 + p.behind_at) & 1) out += p.behind_d;
+        good = good && seq_kb(r) == p.k2 && out < kSeqLimit;
+        r = seq_value(p.k2, out);
+      }
+      s = good ? r : finish_apply_event(sm, e, s);
+      if (kMulti && !(s <= thr)) return false;  // the estimate says so
+    }
+    if (!(s < 3.0e38f)) return false;
+    if (kMulti && lane == 0) sm.ev_sum[e] = s - before;
+  }
+  *sum = s;
+  return true;
+}
+
+// kMulti: some row may be sampled without a crop (the second pass, which costs registers).
+template <typename T, bool kMulti>
 __global__ void __launch_bounds__(kFinThreads, 2) row_finish_kernel(const FinishArgs fa, ExpTable table) {
   extern __shared__ __align__(16) unsigned char finish_smem[];
   FinishShared& sm = *reinterpret_cast<FinishShared*>(finish_smem);
@@ -584,338 +1115,475 @@ __global__ void __launch_bounds__(kFinThreads, 2) row_finish_kernel(const Finish
   }
   const float c1 = __fmul_rn(inv_t, kLog2eHi);
   const RowScale rs = row_scale(mx);
-  auto exact_term = [&](float x) { return expf_ref(__fsub_rn(__fmul_rn(x, inv_t), mx), sm.exp_tab); };
+  // The terms of the sum being formed: e (first pass), or e / sum (multinomial, second pass: the
+  // running cdf of sampler.cpp:58-70, up to the unit in which it passes the coin)
+  float sum = 1.0f, inv_sum = 1.0f, thr = INFINITY;
+  bool probs = false;
+  int hit_unit = 0x7fffffff;  // first unit in which the running sum may pass thr
+  auto exact_term = [&](float x) {
+    const float e = expf_ref(__fsub_rn(__fmul_rn(x, inv_t), mx), sm.exp_tab);
+    return kMulti && probs ? __fdiv_rn(e, sum) : e;
+  };
+  auto scales = [&](uint32_t info, float* lo, float* hi) {
+    unit_scales(rs, mx, unit_ref(info), unit_binade(info), lo, hi);
+    if (kMulti && probs) {  // three more roundings
+      *lo *= inv_sum * (1.0f - 4e-7f);
+      *hi *= inv_sum * (1.0f + 4e-7f);
+    }
+  };
 
   bool decided = head_state >= 0 && fabsf(mx) < 10000.0f;  // block-uniform throughout
   int known = kRowUnknown;
 
-  const bool zero = (rec.z & kUnitZero) != 0u;
-  const bool event = !zero && unit_span(rec.z) != 0u;
-  sm.u.info[tid] = rec.z;
-  sm.u.a0[tid] = (zero || event) ? 0 : (int)rec.x;
-  const unsigned unsure_mask = (zero || event) ? 0u : rec.y;
   bool listing = use_list;
-  int n_groups, n_unsure, n_ev;
+  bool classes = false;  // candidates are counted by value class
+  int n_more = 0;        // lanes that are looked at for candidates in a second round
   float e_floor = INFINITY;
-  int top_level = -1;
   const float cutoff = __fdiv_rn(__fsub_rn(1.0f, mode.topp), (float)(vocab - 1));
-  {
-    if (use_list) {
-      // lanes on every level, and from them the level down to which candidates are listed first: for
-      // top-k the first with at least k lanes (every such lane holds an entry that large, so the k
-      // largest are among what is listed); for top-p as many levels as kFinFirst lanes cover
-      if (tid < kLevels) sm.level_cnt[tid] = 0;
-      __syncthreads();
-      int mine = 0;
-#pragma unroll
-      for (int t = 0; t < kLevels - 1; ++t) {
-        const int c = __reduce_add_sync(0xffffffffu, tid < n_units ? __popc(lanes_up_to(level, t)) : 0);
-        if (lane == t) mine = c;
-      }
-      if (lane < kLevels - 1 && mine > 0) atomicAdd(&sm.level_cnt[lane], mine);
-      __syncthreads();
-      const int upto = lane < kLevels - 1 ? sm.level_cnt[lane] : 0x7fffffff;
-      const unsigned b = __ballot_sync(0xffffffffu, use_topk ? upto >= mode.topk : upto > kFinFirst);
-      top_level = use_topk ? __ffs(b) - 1 : __ffs(b) - 2;  // bit kLevels - 1 is set in any case
-      if (top_level > kLevels - 2) top_level = kLevels - 2;
-      e_floor = top_level >= 0 ? level_floor(top_level) : 2.0f;
-      if (use_topp) e_floor = fmaxf(e_floor, cutoff * 0.999999f);  // the sum is at least 1
-    }
-    // lanes with unsure terms first, then lanes with candidates only
-    unsigned cmask = listing && top_level >= 0 && tid < n_units ? lanes_up_to(level, top_level) & ~unsure_mask : 0u;
-    int tot_u, tot_c;
-    const int pre_u = finish_scan(sm.redi, (__popc(unsure_mask) << 10) | (event ? 1 : 0), &tot_u);
-    const int pre_c = finish_scan(sm.redf_i, __popc(cmask), &tot_c);
-    n_unsure = tot_u >> 10;  // at most 512 events (10 bits) and 16384 lanes
-    n_ev = tot_u & 1023;
-    if (n_unsure + tot_c > kFinGroups) {
-      // candidates all over the row: none is listed here
-      listing = false;
-      cmask = 0u;
-      tot_c = 0;
-    }
-    n_groups = n_unsure + tot_c;
-    if (n_groups > kFinGroups || n_ev > kFinEvents) {
-      decided = false;
-    } else {
-      if (event) sm.ev_unit[pre_u & 1023] = tid;
-      int slot = pre_u >> 10;
-      for (unsigned m = unsure_mask; m != 0u; m &= m - 1u) sm.u.group[slot++] = (uint16_t)(tid * 32 + __ffs(m) - 1);
-      slot = n_unsure + pre_c;
-      for (unsigned m = cmask; m != 0u; m &= m - 1u) sm.u.group[slot++] = (uint16_t)(tid * 32 + __ffs(m) - 1);
-    }
-    if (tid == 0) sm.ev_unit[n_ev < kFinEvents ? n_ev : kFinEvents] = n_units;
-  }
   const float temperature = 1.0f / inv_t;
-  __syncthreads();
-
-  if (decided) {
-    // Half-lanes [32 * task, ...) of the group list, one per thread: which of their logits are
-    // candidates (terms in [lo, hi)) or, for the first n_u groups, unsure; then those terms exactly,
-    // packed, one per lane. By one warp.
-    auto look = [&](int task, int n_g, int n_u, float lo, float hi) {
-      const float x_low = candidate_logit_bound(__logf(lo), mx, temperature);
-      const int h = task * 32 + lane;
-      float x[8];
-      unsigned um = 0u, cm = 0u;
-      int p = 0;
-      if (h < 2 * n_g) {
-        const int g = sm.u.group[h >> 1];
-        const int u = g >> 5;
-        p = u * kUnit + unit_pos(g & 31, h & 1);
-        load8_padded(row, shift, vocab, p, x);
+  for (;;) {
+    const bool zero = (rec.z & kUnitZero) != 0u;
+    const bool event = !zero && (unit_span(rec.z) != 0u || (kMulti && tid >= hit_unit));
+    sm.u.info[tid] = rec.z;
+    sm.u.a0[tid] = (zero || event) ? 0 : (int)rec.x;
+    const unsigned unsure_mask = (zero || event) ? 0u : rec.y;
+    int n_groups, n_unsure, n_ev;
+    int top_level = -1;
+    {
+      if (use_list) {
+        // lanes on every level, and from them the level down to which candidates are listed first: for
+        // top-k the first with at least k lanes (every such lane holds an entry that large, so the k
+        // largest are among what is listed); for top-p as many levels as kFinFirst lanes cover
+        if (tid < kLevels) sm.level_cnt[tid] = 0;
+        __syncthreads();
+        int mine = 0;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) cm |= x[j] >= x_low ? 1u << j : 0u;
-        if ((h >> 1) < n_u) {
-          const uint32_t info = sm.u.info[u];
-          const float r_unit = (float)unit_ref(info);
-          float s_lo, s_hi;
-          unit_scales(rs, mx, unit_ref(info), unit_binade(info), &s_lo, &s_hi);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const float tau = ex2_approx(__fmaf_rn(x[j], c1, -r_unit));
-            if (__float_as_uint(__fmaf_rn(tau, s_lo, kRoundMagic)) != __float_as_uint(__fmaf_rn(tau, s_hi, kRoundMagic)))
-              um |= 1u << j;
-          }
+        for (int t = 0; t < kLevels - 1; ++t) {
+          const int c = __reduce_add_sync(0xffffffffu, tid < n_units ? __popc(lanes_up_to(level, t)) : 0);
+          if (lane == t) mine = c;
         }
+        if (lane < kLevels - 1 && mine > 0) atomicAdd(&sm.level_cnt[lane], mine);
+        __syncthreads();
+        const int upto = lane < kLevels - 1 ? sm.level_cnt[lane] : 0x7fffffff;
+        const unsigned b = __ballot_sync(0xffffffffu, use_topk ? upto >= mode.topk : upto > kFinFirst);
+        top_level = use_topk ? __ffs(b) - 1 : __ffs(b) - 2;  // bit kLevels - 1 is set in any case
+        if (top_level > kLevels - 2) top_level = kLevels - 2;
+        e_floor = top_level >= 0 ? level_floor(top_level) : 2.0f;
+        if (use_topp) e_floor = fmaxf(e_floor, cutoff * 0.999999f);  // the sum is at least 1
       }
-      uint32_t* queue = sm.u.queue[warp];
-      unsigned am = um | cm;
-      float mass = 0.0f;
-      for (;;) {
-        int n_q = __popc(am), inc = n_q;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-          const int o = __shfl_up_sync(0xffffffffu, inc, d);
-          if (lane >= d) inc += o;
-        }
-        const int tot = __shfl_sync(0xffffffffu, inc, 31);
-        if (tot == 0) break;
-        int slot = inc - n_q;
-        while (am != 0u && slot < kFinQueue) {
-          const int j = __ffs(am) - 1;
-          queue[slot++] = (uint32_t)(p + j) | ((cm >> j & 1u) ? kQCand : 0u) | ((um >> j & 1u) ? kQUnsure : 0u);
-          am &= am - 1u;
-        }
-        __syncwarp();
-        const int n_e = tot < kFinQueue ? tot : kFinQueue;
-        for (int e = lane; e < n_e; e += 32) {
-          const uint32_t el = queue[e];
-          const int pe = (int)(el & kQPos), u = pe / kUnit;
-          const float xs = to_f32(row[pe - shift]);
-          const float v = exact_term(xs);
-          if ((el & kQCand) && v >= lo && v < hi) {
-            const int c = atomicAdd(&sm.n_cand, 1);
-            mass += v;
-            if (c < kFinCand) {
-              Entry en;
-              en.key = f32_bits(v);
-              en.idx = pe - shift;
-              sm.cand[c] = en;
-            }
-          }
-          if (el & kQUnsure) {
-            const uint32_t info = sm.u.info[u];
-            float s_lo, s_hi;
-            unit_scales(rs, mx, unit_ref(info), unit_binade(info), &s_lo, &s_hi);
-            const float tau = ex2_approx(__fmaf_rn(xs, c1, -(float)unit_ref(info)));
-            const int approx = (int)(__float_as_uint(__fmaf_rn(tau, s_lo, kRoundMagic)) - kRoundMagicBits);
-            const float t = fminf(__fmul_rn(v, seq_inv_u(unit_binade(info))), 67108864.0f);
-            const float m = rintf(t);
-            if (fabsf(t - m) == 0.5f) {
-              const int c = atomicAdd(&sm.n_tie, 1);
-              if (c < kFinTies) sm.u.tie[c] = (uint32_t)pe | (m > t ? kTieUp : 0u);
-            }
-            const int d = (int)m - approx;
-            if (d != 0) atomicAdd(&sm.u.a0[u], d);
-            if (d & 1) {
-              const int c = atomicAdd(&sm.n_odd, 1);
-              if (c < kFinOdd) sm.u.odd[c] = (uint32_t)pe;
-            }
-          }
-        }
-        __syncwarp();
+      // lanes with unsure terms first, then lanes with candidates only
+      unsigned cmask = listing && top_level >= 0 && tid < n_units ? lanes_up_to(level, top_level) & ~unsure_mask : 0u;
+      int tot_u, tot_c;
+      const int pre_u = finish_scan(sm.redi, (__popc(unsure_mask) << 10) | (event ? 1 : 0), &tot_u);
+      const int pre_c = finish_scan(sm.redf_i, __popc(cmask), &tot_c);
+      n_unsure = tot_u >> 10;  // at most 512 events (10 bits) and 16384 lanes
+      n_ev = tot_u & 1023;
+      if (n_unsure + tot_c > kFinGroups) {
+        // candidates all over the row: none is listed here
+        listing = false;
+        cmask = 0u;
+        tot_c = 0;
       }
-      if (hi > 2.0f) {  // the first pass: the mass listed
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) mass += __shfl_xor_sync(0xffffffffu, mass, d);
-        if (lane == 0 && mass > 0.0f) atomicAdd(&sm.mass, mass);
+      n_groups = n_unsure + tot_c;
+      if (n_groups > kFinGroups || n_ev > kFinEvents) {
+        decided = false;
+      } else {
+        if (event) sm.ev_unit[pre_u & 1023] = tid;
+        int slot = pre_u >> 10;
+        for (unsigned m = unsure_mask; m != 0u; m &= m - 1u) sm.u.group[slot++] = (uint16_t)(tid * 32 + __ffs(m) - 1);
+        slot = n_unsure + pre_c;
+        for (unsigned m = cmask; m != 0u; m &= m - 1u) sm.u.group[slot++] = (uint16_t)(tid * 32 + __ffs(m) - 1);
       }
-    };
-    auto next_task = [&](int* counter) {
-      int task = 0;
-      if (lane == 0) task = atomicAdd(counter, 1);
-      return __shfl_sync(0xffffffffu, task, 0);
-    };
-    // ---- 2. events, a warp each, and the reported lanes; whichever warp is free takes the next task
-    const int n_tasks = n_ev + (2 * n_groups + 31) / 32;
-    for (;;) {
-      const int task = next_task(&sm.n_task);
-      if (task >= n_tasks) break;
-      if (task < n_ev)
-        finish_event(sm, row, shift, vocab, task, exact_term);
-      else
-        look(task - n_ev, n_groups, n_unsure, listing ? e_floor : INFINITY, INFINITY);
+      if (tid == 0) sm.ev_unit[n_ev < kFinEvents ? n_ev : kFinEvents] = n_units;
     }
     __syncthreads();
-    const int n_tie = sm.n_tie, n_odd = sm.n_odd;
-    // Top-p whose nucleus is not in the list yet: the level (and the part of it) down to which the
-    // lanes' largest terms make up for what is missing, a little more to be safe. Those lanes are looked
-    // at while one warp forms the sum.
-    int n_more = 0;
-    float e_more = e_floor;
-    if (use_topp && listing && !(e_floor <= cutoff * head4.z * 0.98f)) {
-      const int upto = lane < kLevels - 1 ? sm.level_cnt[lane] : 0;
-      const int below = __shfl_up_sync(0xffffffffu, upto, 1);
-      const float goal = (mode.topp * 1.002f + 0.003f) * head4.z;
-      const float w = 0.72f * bits_f32((uint32_t)(127 - lane) << 23);  // mean term of a lane on level `lane`
-      const float own = lane > top_level && lane < kLevels - 1 ? (float)(upto - (lane > 0 ? below : 0)) * w : 0.0f;
-      float m = own;
-#pragma unroll
-      for (int d = 1; d < kLevels; d <<= 1) {
-        const float o = __shfl_up_sync(0xffffffffu, m, d);
-        if (lane >= d) m += o;
-      }
-      const float missing = goal - sm.mass;
-      if (missing > 0.0f) {  // block-uniform
-        const unsigned b = __ballot_sync(0xffffffffu, lane < kLevels - 1 && m >= missing * 1.1f);
-        int t = kLevels - 2;
-        float part = 1.0f;
-        if (b != 0u) {
-          t = __ffs(b) - 1;
-          const float in = __shfl_sync(0xffffffffu, m - own, t), of = __shfl_sync(0xffffffffu, own, t);
-          part = fminf((missing * 1.1f - in) / of + 0.1f, 1.0f);
-        }
-        e_more = fmaxf(level_floor(t) * exp2f(1.0f - part), cutoff * 0.999999f);
-        const unsigned gmask = tid < n_units ? lanes_up_to(level, t) : 0u;
-        const int pre = finish_scan(sm.redi, __popc(gmask), &n_more);
-        if (n_more > kFinGroups) {
-          listing = false;
-          n_more = 0;
-        } else {
-          int slot = pre;
-          for (unsigned g = gmask; g != 0u; g &= g - 1u) sm.u.group[slot++] = (uint16_t)(tid * 32 + __ffs(g) - 1);
-        }
-      }
-    }
-    if (n_tie > kFinTies || n_odd > kFinOdd) decided = false;
+
     if (decided) {
-      // ---- exact half-way terms, a warp each. Such a term makes the significand even: it is rounded
-      // up or down by the parity in front of it, i.e. by the parity of the increments since the
-      // half-way term in front of it in the unit (which left the significand even), or since the
-      // unit's start (then the result depends on the parity at which the unit is entered).
-      for (int e = warp; e < n_tie; e += kWarps) {
-        const uint32_t tie = sm.u.tie[e];
-        const int p = (int)(tie & ~kTieUp), u = p / kUnit;
-        int prev = u * kUnit - 1;
-        for (int q = lane; q < n_tie; q += 32) {
-          const int o = (int)(sm.u.tie[q] & ~kTieUp);
-          if (o < p && o > prev) prev = o;
-        }
-        prev = __reduce_max_sync(0xffffffffu, prev);
-        const uint32_t info = sm.u.info[u];
-        const int r_unit = unit_ref(info);
-        float s_lo, s_hi, x[16];
-        unit_scales(rs, mx, r_unit, unit_binade(info), &s_lo, &s_hi);
-        load_unit_lane(row, shift, vocab, u * kUnit, x);
-        unsigned par = 0u;
+      // Half-lanes [32 * task, ...) of the group list, one per thread: which of their logits are
+      // candidates (terms in [lo, hi)) or, for the first n_u groups, unsure; then those terms exactly,
+      // packed, one per lane. By one warp.
+      auto look = [&](int task, int n_g, int n_u, float lo, float hi) {
+        const float x_low = candidate_logit_bound(__logf(lo), mx, temperature);
+        const int h = task * 32 + lane;
+        float x[8];
+        unsigned um = 0u, cm = 0u;
+        int p = 0;
+        if (h < 2 * n_g) {
+          const int g = sm.u.group[h >> 1];
+          const int u = g >> 5;
+          p = u * kUnit + unit_pos(g & 31, h & 1);
+          load8_padded(row, shift, vocab, p, x);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const int pj = u * kUnit + unit_pos(lane, j >> 3) + (j & 7);
-          const float tau = ex2_approx(__fmaf_rn(x[j], c1, -(float)r_unit));
-          const unsigned bits = __float_as_uint(__fmaf_rn(tau, s_lo, kRoundMagic));
-          if (pj > prev && pj < p) par ^= bits;
-        }
-        for (int q = lane; q < n_odd; q += 32) {
-          const int o = (int)sm.u.odd[q];
-          if (o > prev && o < p) par ^= 1u;
-        }
-        par = __popc(__ballot_sync(0xffffffffu, (par & 1u) != 0u)) & 1u;
-        if (lane == 0) {
-          // a0 counts the term rounded to the even one of its two neighbours m; kTieUp: that is the
-          // upper one
-          const int up = (tie & kTieUp) ? 1 : 0;
-          const int c_even = par ? (up ? -1 : 1) : 0, c_odd = par ? 0 : (up ? -1 : 1);
-          if (c_even != 0) atomicAdd(&sm.u.a0[u], c_even);
-          if (prev < u * kUnit) sm.u.a1d[u] = (signed char)(c_odd - c_even);
-        }
-      }
-      __syncthreads();
-      // ---- 3. the runs of ordinary units in front of each event and behind the last
-      for (int e = warp; e <= n_ev; e += kWarps) {
-        const int u0 = e > 0 ? sm.ev_unit[e - 1] + 1 : 0, u1 = sm.ev_unit[e];
-        SeqSummary tot;
-        seq_identity(&tot);
-        int kmin = 255, kmax = 0;
-        for (int ub = u0; ub < u1; ub += 32) {
-          const int u = ub + lane;
-          SeqSummary s;
-          seq_identity(&s);
-          if (u < u1) {
+          for (int j = 0; j < 8; ++j) cm |= x[j] >= x_low ? 1u << j : 0u;
+          if ((h >> 1) < n_u) {
             const uint32_t info = sm.u.info[u];
-            if ((info & kUnitZero) == 0u) {
-              const int k = unit_binade(info);
-              kmin = k < kmin ? k : kmin;
-              kmax = k > kmax ? k : kmax;
-              const uint32_t v = (uint32_t)sm.u.a0[u];
-              s.a0 = v < (uint32_t)kSeqSat ? (int)v : kSeqSat;
-              s.a1 = s.a0 + sm.u.a1d[u];
+            const float r_unit = (float)unit_ref(info);
+            float s_lo, s_hi;
+            scales(info, &s_lo, &s_hi);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              const float tau = ex2_approx(__fmaf_rn(x[j], c1, -r_unit));
+              if (__float_as_uint(__fmaf_rn(tau, s_lo, kRoundMagic)) != __float_as_uint(__fmaf_rn(tau, s_hi, kRoundMagic)))
+                um |= 1u << j;
             }
           }
-          tot = seq_compose(tot, warp_compose(s));
         }
-        kmin = __reduce_min_sync(0xffffffffu, kmin);
-        kmax = __reduce_max_sync(0xffffffffu, kmax);
-        if (lane == 0) {
-          sm.run_a0[e] = tot.a0;
-          sm.run_a1[e] = tot.a1;
-          sm.run_k[e] = kmax == 0 ? 0 : (kmin == kmax ? kmin : -1);
-        }
-      }
-      __syncthreads();
-      // ---- the exact sequential sum, by one warp
-      if (warp == 0) {
-        float s = 0.0f;
-        bool ok = true;
-        for (int e = 0; e <= n_ev && ok; ++e) {
-          const int rk = sm.run_k[e];
-          if (rk != 0) {
-            SeqSummary run;
-            run.a0 = sm.run_a0[e];
-            run.a1 = sm.run_a1[e];
-            const int n = seq_apply(seq_n(s), run);
-            ok = rk == seq_kb(s) && n < kSeqLimit;
-            s = seq_value(rk, n);
-          }
-          if (ok && e < n_ev) {
-            s = e == 0 ? sm.start_sum : finish_apply_event(sm, e, s);
-            ok = s < 3.0e38f;
-          }
-        }
-        if (lane == 0) {
-          sm.sum = s;
-          sm.bad = ok ? 0 : 1;
-          sm.coin = next_coin(&rng);
-        }
-      } else if (n_more > 0) {
+        uint32_t* queue = sm.u.queue[warp];
+        unsigned am = um | cm;
+        float mass = 0.0f;
         for (;;) {
-          const int task = next_task(&sm.n_task2);
-          if (32 * task >= 2 * n_more) break;
-          look(task, n_more, 0, e_more, e_floor);
+          int n_q = __popc(am), inc = n_q;
+#pragma unroll
+          for (int d = 1; d < 32; d <<= 1) {
+            const int o = __shfl_up_sync(0xffffffffu, inc, d);
+            if (lane >= d) inc += o;
+          }
+          const int tot = __shfl_sync(0xffffffffu, inc, 31);
+          if (tot == 0) break;
+          int slot = inc - n_q;
+          while (am != 0u && slot < kFinQueue) {
+            const int j = __ffs(am) - 1;
+            queue[slot++] = (uint32_t)(p + j) | ((cm >> j & 1u) ? kQCand : 0u) | ((um >> j & 1u) ? kQUnsure : 0u);
+            am &= am - 1u;
+          }
+          __syncwarp();
+          const int n_e = tot < kFinQueue ? tot : kFinQueue;
+          for (int e = lane; e < n_e; e += 32) {
+            const uint32_t el = queue[e];
+            const int pe = (int)(el & kQPos), u = pe / kUnit;
+            const float xs = to_f32(row[pe - shift]);
+            const float v = exact_term(xs);
+            if ((el & kQCand) && v >= lo && v < hi) {
+              const int c = atomicAdd(&sm.n_cand, 1);
+              mass += v;
+              if (c < kFinCand) {
+                Entry en;
+                en.key = f32_bits(v);
+                en.idx = pe - shift;
+                sm.cand[c] = en;
+              }
+            }
+            if (el & kQUnsure) {
+              const uint32_t info = sm.u.info[u];
+              float s_lo, s_hi;
+              scales(info, &s_lo, &s_hi);
+              const float tau = ex2_approx(__fmaf_rn(xs, c1, -(float)unit_ref(info)));
+              const int approx = (int)(__float_as_uint(__fmaf_rn(tau, s_lo, kRoundMagic)) - kRoundMagicBits);
+              const float t = fminf(__fmul_rn(v, seq_inv_u(unit_binade(info))), 67108864.0f);
+              const float m = rintf(t);
+              if (fabsf(t - m) == 0.5f) {
+                const int c = atomicAdd(&sm.n_tie, 1);
+                if (c < kFinTies) sm.u.tie[c] = (uint32_t)pe | (m > t ? kTieUp : 0u);
+              }
+              const int d = (int)m - approx;
+              if (d != 0) atomicAdd(&sm.u.a0[u], d);
+              if (d & 1) {
+                const int c = atomicAdd(&sm.n_odd, 1);
+                if (c < kFinOdd) sm.u.odd[c] = (uint32_t)pe;
+              }
+            }
+          }
+          __syncwarp();
         }
+        if (hi > 2.0f) {  // the first pass: the mass listed
+#pragma unroll
+          for (int d = 16; d > 0; d >>= 1) mass += __shfl_xor_sync(0xffffffffu, mass, d);
+          if (lane == 0 && mass > 0.0f) atomicAdd(&sm.mass, mass);
+        }
+      };
+      auto next_task = [&](int* counter) {
+        int task = 0;
+        if (lane == 0) task = atomicAdd(counter, 1);
+        return __shfl_sync(0xffffffffu, task, 0);
+      };
+      // ---- 2. events, a warp each, and the reported lanes; whichever warp is free takes the next task
+      const int n_tasks = n_ev + (2 * n_groups + 31) / 32;
+      for (;;) {
+        const int task = next_task(&sm.n_task);
+        if (task >= n_tasks) break;
+        if (task < n_ev)
+          finish_event(sm, row, shift, vocab, task, exact_term);
+        else
+          look(task - n_ev, n_groups, n_unsure, listing ? e_floor : INFINITY, INFINITY);
       }
       __syncthreads();
-      e_floor = e_more;
-      if (sm.bad) decided = false;
+      const int n_tie = sm.n_tie, n_odd = sm.n_odd;
+      // Top-p whose nucleus is not in the list yet: the level (and the part of it) down to which the
+      // lanes' largest terms make up for what is missing, a little more to be safe. Those lanes are looked
+      // at while one warp forms the sum.
+      n_more = 0;
+      float e_more = e_floor;
+      if (use_topp && listing && !(e_floor <= cutoff * head4.z * 0.98f)) {
+        const int upto = lane < kLevels - 1 ? sm.level_cnt[lane] : 0;
+        const int below = __shfl_up_sync(0xffffffffu, upto, 1);
+        const float goal = (mode.topp * 1.002f + 0.003f) * head4.z;
+        const float w = 0.72f * bits_f32((uint32_t)(127 - lane) << 23);  // mean term of a lane on level `lane`
+        const float own = lane > top_level && lane < kLevels - 1 ? (float)(upto - (lane > 0 ? below : 0)) * w : 0.0f;
+        float m = own;
+#pragma unroll
+        for (int d = 1; d < kLevels; d <<= 1) {
+          const float o = __shfl_up_sync(0xffffffffu, m, d);
+          if (lane >= d) m += o;
+        }
+        const float missing = goal - sm.mass;
+        if (missing > 0.0f) {  // block-uniform
+          const unsigned b = __ballot_sync(0xffffffffu, lane < kLevels - 1 && m >= missing * 1.1f);
+          if (b == 0u) {
+            listing = false;  // not even all levels: a long nucleus
+          } else {
+            const int t = __ffs(b) - 1;
+            const float in = __shfl_sync(0xffffffffu, m - own, t), of = __shfl_sync(0xffffffffu, own, t);
+            const float part = fminf((missing * 1.1f - in) / of + 0.1f, 1.0f);
+            e_more = fmaxf(level_floor(t) * exp2f(1.0f - part), cutoff * 0.999999f);
+            const unsigned gmask = tid < n_units ? lanes_up_to(level, t) : 0u;
+            int slot = finish_scan(sm.redi, __popc(gmask), &n_more);
+            if (n_more > kFinGroups) {
+              listing = false;
+              n_more = 0;
+            } else {
+              for (unsigned g = gmask; g != 0u; g &= g - 1u) sm.u.group[slot++] = (uint16_t)(tid * 32 + __ffs(g) - 1);
+              if (sizeof(T) == 2 && n_more > kFinListLanes) {
+                // counted by value class: no term is evaluated, and there is no limit on how many they are
+                classes = true;
+                for (int q = tid; q < kFinSlots / 2; q += kFinThreads) sm.hist[q] = 0u;
+                if (tid == 0) sm.cls_over = sm.n_counted = sm.n_tiny = 0;
+              }
+            }
+          }
+        }
+      }
+      if (n_tie > kFinTies || n_odd > kFinOdd) decided = false;
+      if (decided) {
+        // ---- exact half-way terms, a warp each. Such a term makes the significand even: it is rounded
+        // up or down by the parity in front of it, i.e. by the parity of the increments since the
+        // half-way term in front of it in the unit (which left the significand even), or since the
+        // unit's start (then the result depends on the parity at which the unit is entered).
+        for (int e = warp; e < n_tie; e += kWarps) {
+          const uint32_t tie = sm.u.tie[e];
+          const int p = (int)(tie & ~kTieUp), u = p / kUnit;
+          int prev = u * kUnit - 1;
+          for (int q = lane; q < n_tie; q += 32) {
+            const int o = (int)(sm.u.tie[q] & ~kTieUp);
+            if (o < p && o > prev) prev = o;
+          }
+          prev = __reduce_max_sync(0xffffffffu, prev);
+          const uint32_t info = sm.u.info[u];
+          const int r_unit = unit_ref(info);
+          float s_lo, s_hi, x[16];
+          scales(info, &s_lo, &s_hi);
+          load_unit_lane(row, shift, vocab, u * kUnit, x);
+          unsigned par = 0u;
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            const int pj = u * kUnit + unit_pos(lane, j >> 3) + (j & 7);
+            const float tau = ex2_approx(__fmaf_rn(x[j], c1, -(float)r_unit));
+            const unsigned bits = __float_as_uint(__fmaf_rn(tau, s_lo, kRoundMagic));
+            if (pj > prev && pj < p) par ^= bits;
+          }
+          for (int q = lane; q < n_odd; q += 32) {
+            const int o = (int)sm.u.odd[q];
+            if (o > prev && o < p) par ^= 1u;
+          }
+          par = __popc(__ballot_sync(0xffffffffu, (par & 1u) != 0u)) & 1u;
+          if (lane == 0) {
+            // a0 counts the term rounded to the even one of its two neighbours m; kTieUp: that is the
+            // upper one
+            const int up = (tie & kTieUp) ? 1 : 0;
+            const int c_even = par ? (up ? -1 : 1) : 0, c_odd = par ? 0 : (up ? -1 : 1);
+            if (c_even != 0) atomicAdd(&sm.u.a0[u], c_even);
+            if (prev < u * kUnit) sm.u.a1d[u] = (signed char)(c_odd - c_even);
+          }
+        }
+        __syncthreads();
+        // ---- 3. the runs of ordinary units in front of each event and behind the last
+        for (int e = warp; e <= n_ev; e += kWarps) {
+          const int u0 = e > 0 ? sm.ev_unit[e - 1] + 1 : 0, u1 = sm.ev_unit[e];
+          SeqSummary tot;
+          seq_identity(&tot);
+          int kmin = 255, kmax = 0;
+          for (int ub = u0; ub < u1; ub += 32) {
+            const int u = ub + lane;
+            SeqSummary s;
+            seq_identity(&s);
+            if (u < u1) {
+              const uint32_t info = sm.u.info[u];
+              if ((info & kUnitZero) == 0u) {
+                const int k = unit_binade(info);
+                kmin = k < kmin ? k : kmin;
+                kmax = k > kmax ? k : kmax;
+                const uint32_t v = (uint32_t)sm.u.a0[u];
+                s.a0 = v < (uint32_t)kSeqSat ? (int)v : kSeqSat;
+                s.a1 = s.a0 + sm.u.a1d[u];
+              }
+            }
+            tot = seq_compose(tot, warp_compose(s));
+          }
+          kmin = __reduce_min_sync(0xffffffffu, kmin);
+          kmax = __reduce_max_sync(0xffffffffu, kmax);
+          if (lane == 0) {
+            sm.run[e] = make_int4(tot.a0, tot.a1, kmax == 0 ? 0 : (kmin == kmax ? kmin : -1), 0);
+          }
+        }
+        __syncthreads();
+        // ---- the exact sequential sum, by one warp
+        if (warp == 0) {
+          int hit = -1;
+          float s = 0.0f;
+          bool ok = finish_replay<kMulti>(sm, n_ev, thr, hit_unit, shift, vocab, &s, &hit);
+          // a cdf that passes the coin nowhere in the units that were looked at, but has units behind them
+          if (probs && hit < 0 && sm.tail_last < n_units - 1) ok = false;
+          if (lane == 0) {
+            if (!probs) {
+              sm.sum = s;
+              sm.coin = next_coin(&rng);
+            }
+            sm.bad = ok ? 0 : 1;
+            sm.tail_pos = hit;  // (-1 but for the multinomial hit)
+          }
+        } else if (classes) {
+          if constexpr (sizeof(T) == 2) {
+            const float x_low = candidate_logit_bound(__logf(e_more), mx, temperature);
+            const ClassSlots slots = class_slots<T>(raw_max);
+            for (;;) {
+              const int task = next_task(&sm.n_task2);
+              if (32 * task >= 2 * n_more) break;
+              const int h = task * 32 + lane;
+              int added = 0;
+              if (h < 2 * n_more) {
+                const int g = sm.u.group[h >> 1];
+                uint32_t w[4];
+                load4_patterns(row, shift, vocab, (g >> 5) * kUnit + unit_pos(g & 31, h & 1), w);
+                auto count = [&](uint32_t pat, float x) {
+                  if (!(x >= x_low)) return;
+                  const uint32_t sl = slots.slot(pat);
+                  if (sl < (uint32_t)kFinSlots) {
+                    atomicAdd(&sm.hist[sl >> 1], 1u << ((sl & 1u) * 16u));
+                    ++added;
+                  } else if (sl == 0x7fffffffu) {
+                    const int k = atomicAdd(&sm.n_tiny, 1);
+                    if (k < kFinTiny) sm.tiny_key[k] = (uint16_t)key_of_pattern16(pat);
+                  } else {
+                    sm.cls_over = 1;
+                  }
+                };
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                  const T* x = reinterpret_cast<const T*>(&w[k]);
+                  count(w[k] & 0xFFFFu, to_f32(x[0]));
+                  count(w[k] >> 16, to_f32(x[1]));
+                }
+              }
+              added = __reduce_add_sync(0xffffffffu, added);
+              if (lane == 0) atomicAdd(&sm.n_counted, added);
+            }
+          }
+        } else if (n_more > 0) {
+          for (;;) {
+            const int task = next_task(&sm.n_task2);
+            if (32 * task >= 2 * n_more) break;
+            look(task, n_more, 0, e_more, e_floor);
+          }
+        }
+        __syncthreads();
+        e_floor = e_more;
+        if (sm.bad) decided = false;
+      }
     }
+    if (!kMulti || !decided || use_list || probs) break;
+    // ---- multinomial: the exact sum is known. Estimates of the cdf behind every unit from the units'
+    // shares of the sum, the binades they leave open, and the units in which the cdf may pass the
+    // coin; then the increments of the units in front of those, as in the sweep, for e / sum.
+    probs = true;
+    sum = sm.sum;
+    inv_sum = __frcp_rn(sum);
+    thr = sm.coin;
+    float* share = reinterpret_cast<float*>(sm.cand);  // (no candidates in this mode)
+    uint32_t* masks = reinterpret_cast<uint32_t*>(sm.cand) + kSwMaxUnits;
+    {
+      const uint32_t v = (uint32_t)sm.u.a0[tid];
+      share[tid] = (zero || event) ? 0.0f : (float)v * bits_f32((uint32_t)(unit_binade(rec.z) - 23) << 23);
+      __syncthreads();
+      if (tid < n_ev) share[sm.ev_unit[tid]] = sm.ev_sum[tid];
+      if (tid == 0) sm.tail_pos = sm.tail_last = n_units - 1;
+      __syncthreads();
+      const float own = share[tid];
+      float inc = own;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const float o = __shfl_up_sync(0xffffffffu, inc, d);
+        if (lane >= d) inc += o;
+      }
+      if (lane == 31) sm.wmass[warp] = inc;
+      __syncthreads();
+      float front = 0.0f;
+      for (int w = 0; w < warp; ++w) front += sm.wmass[w];
+      const float q_in = (front + inc - own) * inv_sum, q_out = (front + inc) * inv_sum;
+      const float margin = sweep_margin((tid + 1) * kUnit);
+      int klo = seq_kb(q_in * (1.0f - margin));
+      const int khi = seq_kb(q_out * (1.0f + margin));
+      uint32_t span = (uint32_t)(khi > klo ? khi - klo : 0);
+      if (span > 62u) span = 62u;
+      if (q_in <= 0.0f || klo < 27) span = kUnitSpanOpen;
+      if (klo < 27) klo = 27;
+      if (tid < n_units && q_out * (1.0f + margin) > thr) atomicMin(&sm.tail_pos, tid);
+      if (tid < n_units && q_out * (1.0f - margin) > thr) atomicMin(&sm.tail_last, tid);
+      __syncthreads();
+      hit_unit = sm.tail_pos;
+      const int last_unit = sm.tail_last;
+      // units behind the last one count as zero: nothing is added there
+      rec.z = (uint32_t)klo | (span << kUnitSpanShift) | (zero || tid > last_unit ? kUnitZero : 0u) | (rec.z & 0xFFFF0000u);
+      sm.u.info[tid] = rec.z;
+      sm.u.a1d[tid] = 0;
+      if (tid == 0) sm.n_task = sm.n_task2 = sm.n_tie = sm.n_odd = 0;
+    }
+    __syncthreads();
+    const int n_sweep = hit_unit < n_units ? hit_unit : n_units;
+    for (int u = warp; u < n_sweep; u += kWarps) {
+      const uint32_t info = sm.u.info[u];
+      if (unit_span(info) != 0u || (info & kUnitZero) != 0u) continue;
+      float s_lo, s_hi, x[16];
+      load_unit_lane(row, shift, vocab, u * kUnit, x);
+      scales(info, &s_lo, &s_hi);
+      const float nr = -(float)unit_ref(info);
+      uint32_t acc = 0u, acc_hi = 0u;
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const float tau = ex2_approx(__fmaf_rn(x[j], c1, nr));
+        acc += __float_as_uint(__fmaf_rn(tau, s_lo, kRoundMagic));
+        acc_hi += __float_as_uint(__fmaf_rn(tau, s_hi, kRoundMagic));
+      }
+      const unsigned unsure = __ballot_sync(0xffffffffu, acc != acc_hi);
+      const unsigned inc = __reduce_add_sync(0xffffffffu, acc);
+      if (lane == 0) {
+        sm.u.a0[u] = (int)(inc - 512u * kRoundMagicBits);
+        masks[u] = unsure;
+      }
+    }
+    __syncthreads();
+    rec.x = (uint32_t)sm.u.a0[tid];
+    rec.y = masks[tid];
+    __syncthreads();
   }
+  if (probs) known = kRowSum;
   if (decided) {
     // ---- 4. the sum is exact: finish on the candidate list, or hand the row on with its sum
-    const float sum = sm.sum, coin = sm.coin;
+    const float coin = sm.coin;
     known = kRowSum;
-    decided = false;
+    sum = sm.sum;
+    decided = probs;
+    if (probs) token = sm.tail_pos >= 0 ? sm.tail_pos : vocab - 1;
     const int n_a = sm.n_cand;
-    if (listing && n_a <= kFinCand) {
+    if (probs) {
+      // decided
+    } else if (classes) {
+      if constexpr (sizeof(T) == 2) {
+        const bool complete = e_floor <= cutoff * sum * 0.999999f;
+        float mass = 0.0f;
+        decided = finish_classes(sm, row, shift, vocab, n_units, n_more, class_slots<T>(raw_max), e_floor, sum, cutoff, mode.topp, complete, coin,
+                                   exact_term, &token, &mass);
+        if (!decided) known = kRowLong;
+      }
+    } else if (listing && n_a <= kFinCand) {
       const bool complete = use_topp && e_floor <= cutoff * sum * 0.999999f;
       float mass;
       decided = finish_tail(sm, e_floor, sum, cutoff, mode.topp, mode.topk, use_topk, complete, coin, &token, &mass);
