@@ -21,14 +21,19 @@ constexpr int kFinThreads = kThreads;   // the tail's helpers are written for kT
 constexpr int kFinEvents = 22;          // event units of a row (2 KB of shared memory each)
 constexpr int kFinTables = 4;           // binades in which an event's terms are summarised
 constexpr int kFinTies = 96;            // exact half-way terms
-constexpr int kFinOdd = 1024;           // corrections that change a parity
 constexpr int kFinGroups = 6144;        // lanes that need another look
 constexpr int kFinCand = 3072;          // candidates
 constexpr int kFinFirst = 256;          // lanes whose candidates are listed at once
-constexpr int kFinSlots = 12288;         // 16-bit logits: value classes counted from the row's maximum down
-constexpr int kFinClasses = 4096;        // ... and how many of them may hold anything
-constexpr int kFinTiny = 64;             // logits close to zero, listed one by one
-constexpr int kFinListLanes = 1536;      // up to this many lanes list their candidates one by one
+constexpr int kFinListLanes = 1536;     // up to this many lanes list their candidates one by one
+constexpr int kFinBins = 4096;          // beyond that they are counted in bins (row_nucleus.cuh)
+constexpr int kFinBinShift = 8;         // positions inside a bin
+constexpr int kLongZones = 120;         // bins whose entries are added one by one
+constexpr int kLongList = 1536;         // entries in those
+constexpr int kNearPart = 376;          // nuclei of up to 16 times as many (a warp's part) are listed by index
+constexpr int kNear = kNearPart * kWarps;
+constexpr int kSampleHalfLanes = 6144;  // of longer rows a sample of this size says where the nucleus ends
+constexpr int kLongTies = 24;           // half-way terms
+constexpr int kLongBinade = 108;        // the lowest binade that a bin is rounded for
 constexpr int kFinQueue = 64;           // a warp's queue of terms to evaluate
 
 // How an event will probably go: the sum enters it in binade k, the lanes in front of lane l (32: all)
@@ -53,59 +58,56 @@ struct FinishTail {
   int idx[kFinCand];
 };
 
-// Its share when the candidates are counted by value class instead of listed.
-struct FinishClasses {
-  uint16_t key[kFinClasses];  // order-preserving keys of the classes that hold candidates, descending
-  uint16_t n[kFinClasses];    // how many
-  float p[kFinClasses];       // their probabilities
-  int ck_kb[kFinClasses / 32 + 1], ck_n[kFinClasses / 32 + 1], ck_pos[kFinClasses / 32 + 1];  // the sum in front of every 32
-  int unit_cnt[kSwMaxUnits];
+// Its share when the candidates are counted in bins (the counts are in FinishShared::hist).
+struct __align__(16) FinishLongFront {
+  uint8_t code[kFinBins];  // 128 + zone, or 1 + binade - kLongBinade
+  alignas(4) uint16_t count[kFinBins];
+  int zone_bin[kLongZones], zone_start[kLongZones], zone_n[kLongZones], zone_fill[kLongZones];
+  int zone_k[kLongZones];         // the binade of the bins in front of a zone
+  uint32_t zone_q[kLongZones];    // increments of all bins in front of it (modulo 2^32)
+  float zone_in[kLongZones];      // the running sum in front of it
+  int4 zone[kLongZones + 1];                        // in order: start, entries, zone_k, zone_q
+  alignas(16) unsigned long long entry[kLongList];  // (probability, inverted index), grouped by zone
+  alignas(16) float sorted[kLongList + 4];          // the probabilities in order
+  uint16_t order[kLongList];                        // of `sorted`
+  uint8_t zone_of[kLongList];
+  int queue_fill[kWarps];
+  int n_tie, tie[kLongTies];
+  int n_near[kWarps];
+};
+struct FinishLong : FinishLongFront {
+  char unused[kFinEvents * kUnit * sizeof(float) - sizeof(FinishLongFront)];
+  uint16_t group_kept[kFinGroups];  // (the group list stays)
+  union {
+    struct {
+      uint32_t queue[kWarps][kFinQueue];
+      int members[kSwMaxUnits];
+    };
+    uint32_t near[kWarps][kNearPart + 64];
+  };
 };
 
-// Slots of the value classes of one row: bit patterns from the largest logit's down, leaving out the
-// patterns of tiny magnitude (the thousands of exponents around zero that no row fills).
-struct ClassSlots {
-  uint32_t tiny, top;  // magnitudes: of the smallest that has a slot, of the row's largest logit
-  bool negative;       // the largest logit is negative
-  // Slot of a pattern; 0x7fffffff for a tiny one, something >= kFinSlots when it is out of range.
-  __device__ __forceinline__ uint32_t slot(uint32_t pat) const {
-    const uint32_t m = pat & 0x7FFFu;
-    if (m < tiny) return 0x7fffffffu;
-    if (!(pat & 0x8000u)) return top - m;
-    return negative ? m - top : (top >= tiny ? top - tiny + 1u : 0u) + (m - tiny);
-  }
-  __device__ __forceinline__ uint32_t pattern(uint32_t slot) const {
-    if (negative) return 0x8000u | (top + slot);
-    const uint32_t pos = top >= tiny ? top - tiny + 1u : 0u;
-    return slot < pos ? top - slot : 0x8000u | (tiny + (slot - pos));
-  }
-  // first slot behind the tiny magnitudes
-  __device__ __forceinline__ uint32_t behind_tiny() const { return negative ? 0u : (top >= tiny ? top - tiny + 1u : 0u); }
+// One row's constants for the passes of row_nucleus.cuh.
+struct LongRow {
+  const void* row;
+  int shift, vocab, n_units;
+  float inv_t, mx, raw_max, c1;
+  // which half-lanes: of every lane, or of the group list
+  int all, n_half;
+  int step;  // every how many-th
+  // the bins (BinMap)
+  float scale;
+  uint32_t limit;
+  float x_lo, x_hi;  // a range of logits
+  // the exact sum; terms are 2^(x c1 - r_row), times s_lo and s_hi in binade kLongBinade
+  float sum, r_row, s_lo, s_hi;
 };
-template <typename T>
-__device__ __forceinline__ ClassSlots class_slots(float raw_max) {
-  ClassSlots c;
-  uint32_t pat;
-  if constexpr (std::is_same<T, __nv_bfloat16>::value) {
-    pat = f32_bits(raw_max) >> 16;
-    c.tiny = (127u - 12u) << 7;  // 2^-12
-  } else {
-    pat = (uint32_t)__half_as_ushort(__float2half_rn(raw_max));
-    c.tiny = (15u - 4u) << 10;  // 2^-4
-  }
-  c.negative = (pat & 0x8000u) != 0u;
-  c.top = pat & 0x7FFFu;
-  if (c.negative && c.top < c.tiny) {  // a tiny negative maximum: slots from the smallest magnitude on
-    c.negative = false;
-    c.top = 0u;
-  }
-  return c;
-}
 
 struct __align__(16) FinishShared {
   static constexpr bool kExt = false;
   static constexpr bool kHasLut = false;
   uint64_t exp_tab[kExpTableSize];
+  LongRow lr;
   float redf[kWarps];
   int redi[kWarps], redf_i[kWarps];
   SeqSummary wsum[3][kWarps];  // seqsum_tile
@@ -119,7 +121,7 @@ struct __align__(16) FinishShared {
   float tail_cum, tail_mass;
   int misc_i[1];
   int level_cnt[kLevels];
-  int n_task, n_task2, n_cand, n_tie, n_odd, bad;
+  int n_task, n_task2, n_cand, n_tie, bad;
   float sum, coin, start_sum, mass;
   int ev_unit[kFinEvents + 1];
   float ev_sum[kFinEvents];  // what each event adds to the sum
@@ -135,23 +137,20 @@ struct __align__(16) FinishShared {
       int tab_inc[kFinEvents][kFinTables][32];       // inclusive sums of the lanes' increments
       signed char tab_d[kFinEvents][kFinTables][32]; // change of a lane's increment when entered odd
       uint32_t tie[kFinTies];                        // padded position | kTieUp
-      uint32_t odd[kFinOdd];                         // padded positions
       uint32_t info[kSwMaxUnits];
       int a0[kSwMaxUnits];                           // increments of the units, entered with an even significand
       signed char a1d[kSwMaxUnits];                  // the same for an odd one, minus a0
       uint32_t queue[kWarps][kFinQueue];   // terms to evaluate exactly: padded position | kQ...
     };
     FinishTail t;
-    FinishClasses c;
+    FinishLong l;
   } u;
   union {
     Entry cand[kFinCand];
-    unsigned hist[kFinSlots / 2];  // 16-bit counters, two per word
+    uint32_t hist[kFinBins];
   };
-  int cls_over, cls_m, n_counted, n_tiny;
-  uint16_t tiny_key[kFinTiny];
 };
-static_assert(sizeof(FinishClasses) <= sizeof(float) * kFinEvents * kUnit, "the group list behind the pool stays");
+static_assert(sizeof(FinishLongFront) < kFinEvents * kUnit * sizeof(float), "the group list stays where it is");
 static_assert(sizeof(FinishShared) <= 115712, "two blocks per SM");
 constexpr uint32_t kTieUp = 1u << 31;
 constexpr uint32_t kQCand = 1u << 31, kQUnsure = 1u << 30, kQPos = (1u << 30) - 1u;
@@ -205,38 +204,6 @@ __device__ __forceinline__ void load_unit_lane(const T* row, int shift, int voca
         x[q * 8 + j] = (i >= 0 && i < vocab) ? to_f32(row[i]) : -INFINITY;
       }
   }
-}
-
-// Eight 16-bit logits as bit patterns, two per word.
-template <typename T>
-__device__ __forceinline__ void load4_patterns(const T* row, int shift, int vocab, int p, uint32_t (&w)[4]) {
-  const int i0 = p - shift;
-  const unsigned short* row16 = reinterpret_cast<const unsigned short*>(row);
-  if (i0 >= 0 && i0 + 8 <= vocab) {
-    const uint4 raw = __ldg(reinterpret_cast<const uint4*>(row16 + i0));
-    w[0] = raw.x;
-    w[1] = raw.y;
-    w[2] = raw.z;
-    w[3] = raw.w;
-  } else {
-    const uint32_t ninf = std::is_same<T, __nv_bfloat16>::value ? 0xFF80u : 0xFC00u;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int i = i0 + 2 * k;
-      const uint32_t lo = i >= 0 && i < vocab ? row16[i] : ninf, hi = i + 1 >= 0 && i + 1 < vocab ? row16[i + 1] : ninf;
-      w[k] = lo | (hi << 16);
-    }
-  }
-}
-// key_of_pattern16 of both halves of a word
-__device__ __forceinline__ uint32_t keys_of_word(uint32_t w) {
-  return w ^ 0x80008000u ^ (((w >> 15) & 0x00010001u) * 0x7FFFu);
-}
-template <typename T>
-__device__ __forceinline__ float value_of_key(uint32_t key) {
-  const uint32_t pat = pattern_of_key16(key);
-  if constexpr (std::is_same<T, __nv_bfloat16>::value) return bits_f32(pat << 16);
-  else return __half2float(__ushort_as_half((unsigned short)pat));
 }
 
 struct FinishArgs {
@@ -632,92 +599,6 @@ __device__ __forceinline__ bool finish_tail(FinishShared& sm, float e_floor, flo
   return true;
 }
 
-// One walk over the value classes [32 * tile, m), from a sum in front of that tile, until the running
-// float sum exceeds thr (by one warp): classes are runs of equal terms with closed-form summaries
-// (class_math.cuh), composed over 32 of them by a scan. Found: *cls, the copy's position in the sorted
-// list, the position of the class's first copy, and the sum there; else the number of entries and
-// their sum. The first walk records the sum in front of every tile.
-__device__ __forceinline__ bool classes_walk(FinishShared& sm, int m, float thr, int tile, int kb, int n, int pos,
-                                             bool record, int* cls, int* at, int* start, float* cum) {
-  const int lane = threadIdx.x & 31;
-  FinishClasses& c = sm.u.c;
-  for (; 32 * tile < m; ++tile) {
-    if (record && lane == 0) {
-      c.ck_kb[tile] = kb;
-      c.ck_n[tile] = n;
-      c.ck_pos[tile] = pos;
-    }
-    const int k = 32 * tile + lane;
-    const float p = k < m ? c.p[k] : 0.0f;
-    const int all = k < m ? (int)c.n[k] : 0;
-    int cnt = all;
-    for (;;) {
-      SeqSummary s = rep_summary(p, cnt, kb);
-      int ic = cnt;
-      const int limit = thr_limit(thr, kb);
-      const bool two = __any_sync(0xffffffffu, s.a0 != s.a1);
-      if (!two) {
-        // the usual tile: nothing in it reaches the limit, and its total is all that is needed
-        const unsigned tot = __reduce_add_sync(0xffffffffu, (unsigned)s.a0);  // at most 32 * 2^26
-        if ((unsigned)n + tot < (unsigned)limit) {
-          n += (int)tot;
-          pos += __reduce_add_sync(0xffffffffu, cnt);
-          break;
-        }
-      }
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        SeqSummary o;
-        o.a0 = __shfl_up_sync(0xffffffffu, s.a0, d);
-        o.a1 = two ? __shfl_up_sync(0xffffffffu, s.a1, d) : o.a0;
-        const int oc = __shfl_up_sync(0xffffffffu, ic, d);
-        if (lane >= d) {
-          s = seq_compose(o, s);
-          ic += oc;
-        }
-      }
-      const int n_out = seq_apply(n, s);
-      const unsigned b = __ballot_sync(0xffffffffu, cnt > 0 && n_out >= limit);
-      if (b == 0u) {
-        n = __shfl_sync(0xffffffffu, n_out, 31);
-        pos += __shfl_sync(0xffffffffu, ic, 31);
-        break;
-      }
-      const int f = __ffs(b) - 1;
-      const int before = __shfl_sync(0xffffffffu, n_out, f > 0 ? f - 1 : 0);
-      WalkState st;
-      st.kb = kb;
-      st.n = f > 0 ? before : n;
-      bool found = false;
-      float sum = 0.0f;
-      int j = 0;
-      if (lane == f) {
-        // a long run may carry the sum through several binades
-        do {
-          j += class_hit_step(&st, p, cnt - j, thr, &found, &sum);
-        } while (!found && j < cnt && seq_apply(st.n, rep_summary(p, cnt - j, st.kb)) >= thr_limit(thr, st.kb));
-      }
-      kb = __shfl_sync(0xffffffffu, st.kb, f);
-      n = __shfl_sync(0xffffffffu, st.n, f);
-      j = __shfl_sync(0xffffffffu, j, f);
-      pos += __shfl_sync(0xffffffffu, ic - cnt, f) + j;
-      const int used = __shfl_sync(0xffffffffu, all - cnt, f) + j;  // copies of class f so far
-      if (__shfl_sync(0xffffffffu, found ? 1 : 0, f)) {
-        *cls = 32 * tile + f;
-        *at = pos - 1;
-        *start = pos - used;
-        *cum = __shfl_sync(0xffffffffu, sum, f);
-        return true;
-      }
-      if (lane < f) cnt = 0;
-      if (lane == f) cnt -= j;
-    }
-  }
-  *at = pos;
-  *cum = seq_value(kb, n);
-  return false;
-}
-
 // Adds the terms of event e to the exact running sum s, looking for the first position at which it
 // exceeds thr (seqsum_warp). p0: position of the event's first term in the row.
 __device__ __forceinline__ bool finish_search_event(FinishShared& sm, int e, float& s, float thr, int p0, int vocab, int* hit) {
@@ -736,193 +617,7 @@ __device__ __forceinline__ bool finish_search_event(FinishShared& sm, int e, flo
   return seqsum_warp<true>(v, s, thr, p0, vocab, hit, &at);
 }
 
-// The rest of sample_topp on the row's value classes (counted in sm.hist and sm.tiny_key): the classes
-// that hold anything with their probabilities, the two walks, and the token of the wanted rank
-// among those of equal probability, by index, with one more look at the lanes that were counted
-// (sm.u.group). Returns as finish_tail.
-template <typename T, typename Term>
-__device__ __forceinline__ bool finish_classes(FinishShared& sm, const T* row, int shift, int vocab, int n_units, int n_groups,
-                                               const ClassSlots& slots, float e_floor, float sum, float cutoff,
-                                               float topp, bool complete, float coin, Term exact_term, int* token,
-                                               float* mass) {
-  constexpr int kPer = kFinSlots / 2 / kFinThreads;  // words per thread
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  FinishClasses& c = sm.u.c;
-  const int n_tiny = sm.n_tiny;
-  if (sm.cls_over || n_tiny > kFinTiny) return false;
-  if (tid == 0) sm.cls_m = 0x7fffffff;
-  // how many classes, and how many logits the counters add up to (a counter that ran over shows)
-  int have = 0, sum_n = 0;
-  unsigned words[kPer];  // 128-bit reads, in distinct banks for eight neighbouring threads
-#pragma unroll
-  for (int k = 0; k < kPer / 4; ++k) {
-    const uint4 q = reinterpret_cast<const uint4*>(sm.hist)[tid * (kPer / 4) + k];
-    words[4 * k] = q.x;
-    words[4 * k + 1] = q.y;
-    words[4 * k + 2] = q.z;
-    words[4 * k + 3] = q.w;
-  }
-#pragma unroll
-  for (int k = 0; k < kPer; ++k) {
-    have += (words[k] & 0xFFFFu ? 1 : 0) + (words[k] >> 16 ? 1 : 0);
-    sum_n += (int)(words[k] & 0xFFFFu) + (int)(words[k] >> 16);
-  }
-  const uint32_t split = slots.behind_tiny();
-  int m, counted;
-  int at0 = finish_scan(sm.redi, have, &m);
-  finish_scan(sm.redf_i, sum_n, &counted);
-  if (counted != sm.n_counted || m + n_tiny > kFinClasses) return false;
-  m += n_tiny;
-#pragma unroll
-  for (int k = 0; k < 2 * kPer; ++k) {
-    const unsigned n = k & 1 ? words[k >> 1] >> 16 : words[k >> 1] & 0xFFFFu;
-    if (n != 0u) {
-      const uint32_t sl = (uint32_t)(tid * 2 * kPer + k);
-      const int o = at0++ + (sl >= split ? n_tiny : 0);
-      c.key[o] = (uint16_t)key_of_pattern16(slots.pattern(sl));
-      c.n[o] = (uint16_t)n;
-      if (sl < split && n_tiny > 0) atomicMax(&sm.tail_pos, o);  // (-1 before)
-    }
-  }
-  __syncthreads();
-  if (tid < n_tiny) {
-    // the tiny ones between the two, largest first
-    const uint16_t mine = sm.tiny_key[tid];
-    int o = sm.tail_pos + 1;
-    for (int k = 0; k < n_tiny; ++k) o += sm.tiny_key[k] > mine || (sm.tiny_key[k] == mine && k < tid) ? 1 : 0;
-    c.key[o] = mine;
-    c.n[o] = 1;
-  }
-  __syncthreads();
-  for (int k = tid; k < m; k += kFinThreads) {
-    const float e = exact_term(value_of_key<T>(c.key[k]));
-    const float p = __fdiv_rn(e, sum);
-    c.p[k] = p;
-    // the crop (sampler.cpp:136-143): nothing below is a candidate; and below the floor not everything
-    // was counted
-    if (p < cutoff || e < e_floor) atomicMin(&sm.cls_m, k);
-  }
-  c.unit_cnt[tid] = 0;
-  __syncthreads();
-  if (sm.cls_m < m) m = sm.cls_m;
-  if (warp == 0) {
-    int cls = 0, at = 0, start = 0, n_tiles = (m + 31) / 32;
-    float cum = 0.0f;
-    const bool found = classes_walk(sm, m, topp, 0, 1, 0, 0, true, &cls, &at, &start, &cum);
-    bool ok = m > 0 && (found || complete);
-    if (found) {
-      n_tiles = cls / 32 + 1;
-    } else if (m > 0) {
-      cls = m - 1;  // the sum never exceeded topp: everything is kept (sampler.cpp:152)
-      start = at - (int)c.n[cls];
-      at -= 1;
-    }
-    const float r = __fmul_rn(coin, cum);  // sampler.cpp:162
-    if (ok && r < cum) {
-      __syncwarp();
-      int t = 0;
-      for (int q = lane; q < n_tiles; q += 32)
-        if (seq_value(c.ck_kb[q], c.ck_n[q]) <= r) t = q;
-      t = __reduce_max_sync(0xffffffffu, t);
-      int cls2 = 0, at2 = 0, start2 = 0;
-      float cum2;
-      if (classes_walk(sm, m, r, t, c.ck_kb[t], c.ck_n[t], c.ck_pos[t], false, &cls2, &at2, &start2, &cum2) && at2 <= at) {
-        cls = cls2;
-        at = at2;
-        start = start2;
-      }
-    }
-    if (lane == 0) {
-      // classes of the same float probability are one group, in index order
-      int g0 = cls, g1 = cls, rank = at - start;
-      if (ok) {
-        const float p = c.p[cls];
-        while (g0 > 0 && c.p[g0 - 1] == p) rank += (int)c.n[--g0];
-        while (g1 + 1 < m && c.p[g1 + 1] == p) ++g1;
-      }
-      sm.tail_last = ok ? (int)c.key[g0] : -1;  // the group's keys
-      sm.tail_bin = ok ? (int)c.key[g1] : -1;
-      sm.tail_cnt = rank;
-      sm.tail_mass = cum;
-    }
-  }
-  __syncthreads();
-  *mass = sm.tail_mass;
-  if (sm.tail_last < 0) return false;
-  const uint32_t g_lo = (uint32_t)sm.tail_bin, span = (uint32_t)(sm.tail_last - sm.tail_bin);
-  const int rank = sm.tail_cnt;
-  for (int h0 = tid; h0 < 2 * n_groups; h0 += 4 * kFinThreads) {
-    uint32_t w[4][4];
-    int unit[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {  // four reads of the row in flight
-      const int h = h0 + q * kFinThreads;
-      unit[q] = -1;
-      if (h < 2 * n_groups) {
-        const int g = sm.u.group[h >> 1];
-        unit[q] = g >> 5;
-        load4_patterns(row, shift, vocab, unit[q] * kUnit + unit_pos(g & 31, h & 1), w[q]);
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      if (unit[q] < 0) continue;
-      int n = 0;
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const uint32_t key = keys_of_word(w[q][k]);
-        n += ((key & 0xFFFFu) - g_lo <= span ? 1 : 0) + ((key >> 16) - g_lo <= span ? 1 : 0);
-      }
-      if (n > 0) atomicAdd(&c.unit_cnt[unit[q]], n);
-    }
-  }
-  if (tid == 0) sm.tail_pos = -1;
-  __syncthreads();
-  int tot;
-  const int mine = tid < n_units ? c.unit_cnt[tid] : 0;
-  const int pre = finish_scan(sm.redf_i, mine, &tot);
-  if (rank >= pre && rank < pre + mine) {
-    sm.tail_bin = tid;
-    sm.tail_cnt = rank - pre;
-    sm.tail_pos = 0;
-  }
-  __syncthreads();
-  if (sm.tail_pos < 0) return false;
-  if (warp == 0) {
-    const int u = sm.tail_bin;
-    int left = sm.tail_cnt;
-    int found = -1;
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      uint32_t w[4];
-      load4_patterns(row, shift, vocab, u * kUnit + unit_pos(lane, q), w);
-      unsigned in = 0u;  // this lane's members among its eight logits
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const uint32_t key = keys_of_word(w[k]);
-        in |= ((key & 0xFFFFu) - g_lo <= span ? 1u : 0u) << (2 * k);
-        in |= ((key >> 16) - g_lo <= span ? 1u : 0u) << (2 * k + 1);
-      }
-      const int n = __popc(in);
-      int inc = n;
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const int o = __shfl_up_sync(0xffffffffu, inc, d);
-        if (lane >= d) inc += o;
-      }
-      if (left >= inc - n && left < inc) {
-        for (int k = left - (inc - n); k > 0; --k) in &= in - 1u;
-        found = u * kUnit + unit_pos(lane, q) + __ffs(in) - 1 - shift;
-      }
-      left -= __shfl_sync(0xffffffffu, inc, 31);
-    }
-    found = __reduce_max_sync(0xffffffffu, found);
-    if (lane == 0) sm.tail_pos = found;
-  }
-  __syncthreads();
-  *token = sm.tail_pos;
-  return true;
-}
+#include "row_nucleus.cuh"
 
 // Lane e: the plan of event e, from the sum in front of it as the runs and events in front of it
 // estimate it (good to a few hundred units of the last place; a lane's increments are thousands).
@@ -1061,7 +756,7 @@ __global__ void __launch_bounds__(kFinThreads, 2) row_finish_kernel(const Finish
   if (tid < kExpTableSize) sm.exp_tab[tid] = table.t[tid];
   sm.u.a1d[tid] = 0;
   if (tid == 0) sm.mass = 0.0f;
-  if (tid == 0) sm.n_task = sm.n_task2 = sm.n_cand = sm.n_tie = sm.n_odd = sm.bad = 0;
+  if (tid == 0) sm.n_task = sm.n_task2 = sm.n_cand = sm.n_tie = sm.bad = 0;
   grid_dependency_wait();  // the sweep's records are complete and visible from here on
 
   // ---- 1. the unit records (the row's head and RNG state meanwhile). Past the L1 cache: a block that
@@ -1114,6 +809,18 @@ __global__ void __launch_bounds__(kFinThreads, 2) row_finish_kernel(const Finish
     return;
   }
   const float c1 = __fmul_rn(inv_t, kLog2eHi);
+  if (use_list && tid == 0) {
+    LongRow& lr = sm.lr;
+    lr.row = row;
+    lr.shift = shift;
+    lr.vocab = vocab;
+    lr.n_units = n_units;
+    lr.inv_t = inv_t;
+    lr.mx = mx;
+    lr.raw_max = raw_max;
+    lr.c1 = c1;
+    lr.step = 1;
+  }
   const RowScale rs = row_scale(mx);
   // The terms of the sum being formed: e (first pass), or e / sum (multinomial, second pass: the
   // running cdf of sampler.cpp:58-70, up to the unit in which it passes the coin)
@@ -1136,9 +843,9 @@ __global__ void __launch_bounds__(kFinThreads, 2) row_finish_kernel(const Finish
   int known = kRowUnknown;
 
   bool listing = use_list;
-  bool classes = false;  // candidates are counted by value class
+  bool counted = false, all_lanes = false;  // candidates are counted in bins; those of every lane
   int n_more = 0;        // lanes that are looked at for candidates in a second round
-  float e_floor = INFINITY;
+  float e_floor = INFINITY, list_floor = INFINITY;
   const float cutoff = __fdiv_rn(__fsub_rn(1.0f, mode.topp), (float)(vocab - 1));
   const float temperature = 1.0f / inv_t;
   for (;;) {
@@ -1181,6 +888,7 @@ __global__ void __launch_bounds__(kFinThreads, 2) row_finish_kernel(const Finish
       if (n_unsure + tot_c > kFinGroups) {
         // candidates all over the row: none is listed here
         listing = false;
+        e_floor = INFINITY;
         cmask = 0u;
         tot_c = 0;
       }
@@ -1277,10 +985,6 @@ __global__ void __launch_bounds__(kFinThreads, 2) row_finish_kernel(const Finish
               }
               const int d = (int)m - approx;
               if (d != 0) atomicAdd(&sm.u.a0[u], d);
-              if (d & 1) {
-                const int c = atomicAdd(&sm.n_odd, 1);
-                if (c < kFinOdd) sm.u.odd[c] = (uint32_t)pe;
-              }
             }
           }
           __syncwarp();
@@ -1307,7 +1011,7 @@ __global__ void __launch_bounds__(kFinThreads, 2) row_finish_kernel(const Finish
           look(task - n_ev, n_groups, n_unsure, listing ? e_floor : INFINITY, INFINITY);
       }
       __syncthreads();
-      const int n_tie = sm.n_tie, n_odd = sm.n_odd;
+      const int n_tie = sm.n_tie;
       // Top-p whose nucleus is not in the list yet: the level (and the part of it) down to which the
       // lanes' largest terms make up for what is missing, a little more to be safe. Those lanes are looked
       // at while one warp forms the sum.
@@ -1329,7 +1033,7 @@ __global__ void __launch_bounds__(kFinThreads, 2) row_finish_kernel(const Finish
         if (missing > 0.0f) {  // block-uniform
           const unsigned b = __ballot_sync(0xffffffffu, lane < kLevels - 1 && m >= missing * 1.1f);
           if (b == 0u) {
-            listing = false;  // not even all levels: a long nucleus
+            listing = false;  // not even all levels
           } else {
             const int t = __ffs(b) - 1;
             const float in = __shfl_sync(0xffffffffu, m - own, t), of = __shfl_sync(0xffffffffu, own, t);
@@ -1342,17 +1046,26 @@ __global__ void __launch_bounds__(kFinThreads, 2) row_finish_kernel(const Finish
               n_more = 0;
             } else {
               for (unsigned g = gmask; g != 0u; g &= g - 1u) sm.u.group[slot++] = (uint16_t)(tid * 32 + __ffs(g) - 1);
-              if (sizeof(T) == 2 && n_more > kFinListLanes) {
-                // counted by value class: no term is evaluated, and there is no limit on how many they are
-                classes = true;
-                for (int q = tid; q < kFinSlots / 2; q += kFinThreads) sm.hist[q] = 0u;
-                if (tid == 0) sm.cls_over = sm.n_counted = sm.n_tiny = 0;
-              }
+              if (n_more > kFinListLanes) counted = true;
             }
           }
         }
       }
-      if (n_tie > kFinTies || n_odd > kFinOdd) decided = false;
+      if (use_topp && !listing) {
+        // a nucleus all over the row: whatever passes the crop
+        counted = all_lanes = true;
+        e_more = cutoff * head4.z * 0.98f;
+      }
+      if (counted) {
+        if (tid == 0) {
+          set_bins(sm.lr, candidate_logit_bound(__logf(e_more), mx, temperature));
+          sm.lr.all = all_lanes ? 1 : 0;
+          sm.lr.n_half = all_lanes ? n_units * (kUnit / 8) : 2 * n_more;
+          sm.lr.step = (sm.lr.n_half + kSampleHalfLanes - 1) / kSampleHalfLanes;
+        }
+        for (int q = tid; q < kFinBins; q += kFinThreads) sm.hist[q] = 0u;
+      }
+      if (n_tie > kFinTies) decided = false;
       if (decided) {
         // ---- exact half-way terms, a warp each. Such a term makes the significand even: it is rounded
         // up or down by the parity in front of it, i.e. by the parity of the increments since the
@@ -1372,17 +1085,24 @@ __global__ void __launch_bounds__(kFinThreads, 2) row_finish_kernel(const Finish
           float s_lo, s_hi, x[16];
           scales(info, &s_lo, &s_hi);
           load_unit_lane(row, shift, vocab, u * kUnit, x);
-          unsigned par = 0u;
+          unsigned par = 0u, um = 0u;
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
             const int pj = u * kUnit + unit_pos(lane, j >> 3) + (j & 7);
             const float tau = ex2_approx(__fmaf_rn(x[j], c1, -(float)r_unit));
-            const unsigned bits = __float_as_uint(__fmaf_rn(tau, s_lo, kRoundMagic));
-            if (pj > prev && pj < p) par ^= bits;
+            const unsigned lo = __float_as_uint(__fmaf_rn(tau, s_lo, kRoundMagic));
+            const unsigned hi = __float_as_uint(__fmaf_rn(tau, s_hi, kRoundMagic));
+            if (pj > prev && pj < p) {
+              par ^= lo;
+              um |= lo != hi ? 1u << j : 0u;
+            }
           }
-          for (int q = lane; q < n_odd; q += 32) {
-            const int o = (int)sm.u.odd[q];
-            if (o > prev && o < p) par ^= 1u;
+          for (; um != 0u; um &= um - 1u) {  // the unsure ones exactly
+            const int j = __ffs(um) - 1;
+            const float xs = to_f32(row[u * kUnit + unit_pos(lane, j >> 3) + (j & 7) - shift]);
+            const float tau = ex2_approx(__fmaf_rn(xs, c1, -(float)r_unit));
+            const float t = fminf(__fmul_rn(exact_term(xs), seq_inv_u(unit_binade(info))), 67108864.0f);
+            par ^= __float_as_uint(__fmaf_rn(tau, s_lo, kRoundMagic)) ^ (unsigned)(int)rintf(t);
           }
           par = __popc(__ballot_sync(0xffffffffu, (par & 1u) != 0u)) & 1u;
           if (lane == 0) {
@@ -1440,43 +1160,8 @@ __global__ void __launch_bounds__(kFinThreads, 2) row_finish_kernel(const Finish
             sm.bad = ok ? 0 : 1;
             sm.tail_pos = hit;  // (-1 but for the multinomial hit)
           }
-        } else if (classes) {
-          if constexpr (sizeof(T) == 2) {
-            const float x_low = candidate_logit_bound(__logf(e_more), mx, temperature);
-            const ClassSlots slots = class_slots<T>(raw_max);
-            for (;;) {
-              const int task = next_task(&sm.n_task2);
-              if (32 * task >= 2 * n_more) break;
-              const int h = task * 32 + lane;
-              int added = 0;
-              if (h < 2 * n_more) {
-                const int g = sm.u.group[h >> 1];
-                uint32_t w[4];
-                load4_patterns(row, shift, vocab, (g >> 5) * kUnit + unit_pos(g & 31, h & 1), w);
-                auto count = [&](uint32_t pat, float x) {
-                  if (!(x >= x_low)) return;
-                  const uint32_t sl = slots.slot(pat);
-                  if (sl < (uint32_t)kFinSlots) {
-                    atomicAdd(&sm.hist[sl >> 1], 1u << ((sl & 1u) * 16u));
-                    ++added;
-                  } else if (sl == 0x7fffffffu) {
-                    const int k = atomicAdd(&sm.n_tiny, 1);
-                    if (k < kFinTiny) sm.tiny_key[k] = (uint16_t)key_of_pattern16(pat);
-                  } else {
-                    sm.cls_over = 1;
-                  }
-                };
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                  const T* x = reinterpret_cast<const T*>(&w[k]);
-                  count(w[k] & 0xFFFFu, to_f32(x[0]));
-                  count(w[k] >> 16, to_f32(x[1]));
-                }
-              }
-              added = __reduce_add_sync(0xffffffffu, added);
-              if (lane == 0) atomicAdd(&sm.n_counted, added);
-            }
-          }
+        } else if (counted) {
+          bin_count<T>(sm, warp - 1, kWarps - 1);
         } else if (n_more > 0) {
           for (;;) {
             const int task = next_task(&sm.n_task2);
@@ -1485,6 +1170,7 @@ __global__ void __launch_bounds__(kFinThreads, 2) row_finish_kernel(const Finish
           }
         }
         __syncthreads();
+        list_floor = e_floor;
         e_floor = e_more;
         if (sm.bad) decided = false;
       }
@@ -1534,7 +1220,7 @@ __global__ void __launch_bounds__(kFinThreads, 2) row_finish_kernel(const Finish
       rec.z = (uint32_t)klo | (span << kUnitSpanShift) | (zero || tid > last_unit ? kUnitZero : 0u) | (rec.z & 0xFFFF0000u);
       sm.u.info[tid] = rec.z;
       sm.u.a1d[tid] = 0;
-      if (tid == 0) sm.n_task = sm.n_task2 = sm.n_tie = sm.n_odd = 0;
+      if (tid == 0) sm.n_task = sm.n_task2 = sm.n_tie = 0;
     }
     __syncthreads();
     const int n_sweep = hit_unit < n_units ? hit_unit : n_units;
@@ -1573,27 +1259,20 @@ __global__ void __launch_bounds__(kFinThreads, 2) row_finish_kernel(const Finish
     decided = probs;
     if (probs) token = sm.tail_pos >= 0 ? sm.tail_pos : vocab - 1;
     const int n_a = sm.n_cand;
-    if (probs) {
-      // decided
-    } else if (classes) {
-      if constexpr (sizeof(T) == 2) {
-        const bool complete = e_floor <= cutoff * sum * 0.999999f;
-        float mass = 0.0f;
-        decided = finish_classes(sm, row, shift, vocab, n_units, n_more, class_slots<T>(raw_max), e_floor, sum, cutoff, mode.topp, complete, coin,
-                                   exact_term, &token, &mass);
-        if (!decided) known = kRowLong;
+    if (!probs && use_list) {
+      if (!counted && listing && n_a <= kFinCand) {
+        const bool complete = use_topp && e_floor <= cutoff * sum * 0.999999f;
+        float mass;
+        decided = finish_tail(sm, e_floor, sum, cutoff, mode.topp, mode.topk, use_topk, complete, coin, &token, &mass);
       }
-    } else if (listing && n_a <= kFinCand) {
-      const bool complete = use_topp && e_floor <= cutoff * sum * 0.999999f;
-      float mass;
-      decided = finish_tail(sm, e_floor, sum, cutoff, mode.topp, mode.topk, use_topk, complete, coin, &token, &mass);
-      // every token that is not listed has e < e_floor, so a nucleus that the list does not hold
-      // needs at least (missing mass) / e_floor more of them
-      if (!decided && use_topp && !complete &&
-          (float)n_a + (mode.topp - mass) * sum / e_floor > (float)kVcMinNucleus)
-        known = kRowLong;
-    } else if (use_topp) {
-      known = kRowLong;
+      if (!decided) {
+        __syncthreads();
+        if (!counted && tid == 0) sm.lr.all = 1;
+        token = finish_long<T>(sm, counted, n_more, e_floor, list_floor, sm.mass, sum, cutoff, mode.topp, mode.topk,
+                            use_topk, coin);
+        decided = token >= 0;
+      }
+      if (!decided) known = kRowLong;
     }
   }
   if (decided) {
