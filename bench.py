@@ -42,8 +42,10 @@ NBUF = 4  # rotating input buffers: 4 x 65.7 MB > 126 MB of L2
 FALLBACK_HBM_GBS = 6650.0
 
 PARITY_ROWS = 64
-KERNEL_SOURCES = ["executorch_b200/csrc/sampler_kernels.cu", "executorch_b200/csrc/guided_sum.cuh",
-                  "executorch_b200/csrc/cluster_topp.cuh", "executorch_b200/csrc/cluster_math.cuh",
+KERNEL_SOURCES = ["executorch_b200/csrc/sampler_kernels.cu", "executorch_b200/csrc/sampler_device.cuh",
+                  "executorch_b200/csrc/fast_path.cu", "executorch_b200/csrc/row_sweep.cuh",
+                  "executorch_b200/csrc/row_finish.cuh", "executorch_b200/csrc/row_nucleus.cuh",
+                  "executorch_b200/csrc/cluster_math.cuh",
                   "executorch_b200/csrc/exact_math.cuh", "executorch_b200/csrc/class_math.cuh",
                   "executorch_b200/csrc/value_class_tail.cuh"]
 

@@ -249,10 +249,8 @@ etb200_error_t sample_rows_device(
   if (rows == 0 && peers.epoch == 0ull) return ETB200_OK;
   if (h->inv_temperature == 0.0f || rows == 0) {
     // greedy: no coin is drawn and the RNG state does not move (sampler.cpp:226-228)
-    int blocks = (int)(rows < (int64_t)h->sm_count * 4 ? rows : (int64_t)h->sm_count * 4);
-    if (blocks < 1) blocks = 1;
     ETB_CUDA(launch_argmax_rows(rows == 0 ? kDtypeFloat : dtype, logits, rows, h->vocab, row_stride, out_ids, peers,
-                                blocks, h->d_status, stream));
+                                h->sm_count, h->d_status, stream));
     h->launches += 1;
     return ETB200_OK;
   }

@@ -44,7 +44,6 @@ cudaError_t launch_sweep_t(const SweepArgs& args, int csize, int sm_count, cudaS
     if (e != cudaSuccess) return e;
     if (n_cl < 1) n_cl = 1;
     resident[csize].store(n_cl, std::memory_order_relaxed);
-
   }
   const int64_t n = args.rows < n_cl ? args.rows : n_cl;
   cfg.gridDim = dim3((unsigned)(n * csize), 1, 1);

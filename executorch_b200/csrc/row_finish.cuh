@@ -1,6 +1,6 @@
 // Second kernel of the fast sampling path: one block per row turns what row_sweep.cuh left into the
 // exact softmax sum and, for a nucleus (or top-k set) that fits the block's lists, into the token.
-// Included by sampler_kernels.cu inside its unnamed namespace (uses its helpers).
+// Included by fast_path.cu inside its unnamed namespace (uses its helpers).
 //
 //   1. the row's unit records: which units are "events" (the running sum may leave its binade
 //      there, or the row starts there), which lanes need another look

@@ -1,5 +1,5 @@
 // First of the two kernels of the fast sampling path: one streaming sweep over the logits.
-// Included by sampler_kernels.cu inside its unnamed namespace (uses its helpers).
+// Included by fast_path.cu inside its unnamed namespace (uses its helpers).
 //
 // The reference adds the softmax denominator in index order in float (sampler.cpp:198-203), and
 // its tokens depend on every rounding of that sum. While the running sum stays in one binade
@@ -182,12 +182,6 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
 __device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
   f32x2 r;
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-
-__device__ __forceinline__ float warp_max_f32(float v) {
-  float r;
-  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
   return r;
 }
 
@@ -475,7 +469,6 @@ __global__ void __launch_bounds__(kSwThreads, SweepLayout<T, kUnitsPerWarp>::kBl
       // what does not need the others' word
       const float margin = sweep_margin(pos0 + (lane + 1) * kUnit);
       const float m_lo = 1.0f - margin, m_hi = 1.0f + margin;
-      
       const bool ok = wait_bulk_copy(&sm.told[par], told_phase);
       // every lane: its unit's plan
       SweepExchange x;

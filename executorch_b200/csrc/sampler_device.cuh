@@ -639,6 +639,12 @@ __device__ __forceinline__ bool head_sum(
   return hit;
 }
 
+__device__ __forceinline__ float warp_max_f32(float v) {
+  float r;
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+
 // Writes the token of row r: to out_ids[r], or -- when peer buffers are given -- straight into
 // every listed buffer at [offset + r] (each may live on another GPU of the node: plain
 // stores over NVLink, one thread per destination). Block-uniform `token`.

@@ -572,110 +572,151 @@ __global__ void __launch_bounds__(kThreads, 2) sample_rows_kernel(
 // index order: the lowest index among equal maxima wins, -0 equals +0, a NaN never
 // replaces the running maximum, and a NaN in element 0 is never replaced.
 // ---------------------------------------------------------------------------------------
-// Each thread keeps eight 128-bit loads in flight per iteration, each of them contiguous
-// across the warp: with one block per row and fewer than two blocks per SM at batch 256, the
-// bytes in flight decide the bandwidth.
+//
+// Bound by HBM: every logit is read once. A cluster of blocks shares a row, so that small batches
+// fill the chip, and the partial maxima meet in the first block's shared memory. A thread keeps eight 128-bit loads in flight, contiguous across the
+// warp. A vector costs its packed maximum, a comparison and two selects; which of its elements it
+// was is looked up for the winning vector alone. Vectors start at the 16-byte boundary at or in
+// front of the row's first logit, whatever the row's alignment. Measured against one block per row with a
+// comparison per logit and scalar loads for unaligned rows: one row of 128256 bf16 8.2 -> 3.7 us,
+// 64 x 50257 fp16 10.3 -> 5.2 us, 256 x 128256 bf16 14.6 -> 13.1 us (5.0 TB/s).
 constexpr int kArgVecs = 8;
+constexpr int kArgMaxCluster = 16;
 
-template <typename T, bool kRawU16>
-__global__ void __launch_bounds__(kThreads, 2) argmax_rows_kernel(
+template <typename T>
+__device__ __forceinline__ float arg_value(T x) {
+  if constexpr (std::is_same<T, unsigned short>::value) return (float)x;  // sample<uint16_t> compares the raw integers
+  else return to_f32(x);
+}
+
+// Largest value of a vector; NaNs count only if there is nothing else.
+template <typename T>
+__device__ __forceinline__ float vec_max(const uint4& raw) {
+  if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+    const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&raw);
+    const __nv_bfloat162 m = __hmax2(__hmax2(p[0], p[1]), __hmax2(p[2], p[3]));
+    return fmaxf(__bfloat162float(m.x), __bfloat162float(m.y));
+  } else if constexpr (std::is_same<T, __half>::value) {
+    const __half2* p = reinterpret_cast<const __half2*>(&raw);
+    const __half2 m = __hmax2(__hmax2(p[0], p[1]), __hmax2(p[2], p[3]));
+    return fmaxf(__half2float(m.x), __half2float(m.y));
+  } else if constexpr (std::is_same<T, float>::value) {
+    return fmaxf(fmaxf(__uint_as_float(raw.x), __uint_as_float(raw.y)),
+                 fmaxf(__uint_as_float(raw.z), __uint_as_float(raw.w)));
+  } else {
+    const unsigned m = __vmaxu2(__vmaxu2(raw.x, raw.y), __vmaxu2(raw.z, raw.w));
+    return (float)max(m & 0xFFFFu, m >> 16);
+  }
+}
+
+// The lanes' largest value and the lowest vector that holds it, in every lane.
+__device__ __forceinline__ void arg_reduce(float* best, int* v) {
+  const float m = warp_max_f32(*best);
+  *v = __reduce_min_sync(0xffffffffu, *best == m ? *v : 0x7fffffff);
+  *best = m;
+}
+
+template <typename T, int kArgThreads>
+__global__ void __launch_bounds__(kArgThreads, 1024 / kArgThreads) argmax_rows_kernel(
     const T* __restrict__ logits, int64_t rows, int vocab, int64_t row_stride,
     int64_t* __restrict__ out_ids, PeerOut peers, int* __restrict__ status) {
   constexpr int kPerVec = 16 / sizeof(T);
-  __shared__ float sv[kWarps];
-  __shared__ int si[kWarps];
+  constexpr int kArgWarps = kArgThreads / 32;
+  __shared__ float sv[kArgWarps], cv[kArgMaxCluster];
+  __shared__ int si[kArgWarps], ci[kArgMaxCluster];
+  __shared__ int answer;
+  const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const int csize = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {
+  grid_launch_dependents();
+  grid_dependency_wait();
+  // (no row at all in a launch that only takes part in the arrival barrier)
+  for (int64_t r = blockIdx.x / csize; r < rows; r += gridDim.x / csize) {
     const T* row = logits + r * row_stride;
-    const bool vec_ok = (reinterpret_cast<uintptr_t>(row) & 15u) == 0;
-    const uint4* row4 = reinterpret_cast<const uint4*>(row);
-    const int nvec = vec_ok ? vocab / kPerVec : 0;
+    const int shift = (int)((reinterpret_cast<uintptr_t>(row) & 15u) / sizeof(T));
+    const uint4* base4 = reinterpret_cast<const uint4*>(row - shift);
+    // vectors [0, nvec) cover the row; [full0, full1) hold nothing but logits
+    const int nvec = (int)(((int64_t)shift + vocab + kPerVec - 1) / kPerVec);
+    const int full0 = shift > 0 ? 1 : 0, full1 = (int)(((int64_t)shift + vocab) / kPerVec);
+    const int per = (nvec + csize - 1) / csize;
+    const int beg = max(rank * per, full0), end = min((rank + 1) * per, full1);
     float best = -INFINITY;
-    int besti = 0x7fffffff;  // "nothing better than -inf seen": resolved to the first index below
-    // A thread visits its elements in increasing index order (vector q * kThreads + tid of
-    // each group, then the ragged tail), so strict '>' keeps its lowest index of a maximum.
-    for (int v0 = 0; v0 < nvec; v0 += kThreads * kArgVecs) {
+    int bestv = 0x7fffffff;  // "nothing better than -inf seen"
+    // A thread visits its vectors in increasing order, so strict '>' keeps the first of equal ones.
+    for (int v0 = beg; v0 < end; v0 += kArgThreads * kArgVecs) {
       uint4 raw[kArgVecs];
 #pragma unroll
       for (int q = 0; q < kArgVecs; ++q) {
-        const int v = v0 + q * kThreads + tid;
-        if (v < nvec) raw[q] = __ldg(row4 + v);
+        const int v = v0 + q * kArgThreads + tid;
+        if (v < end) raw[q] = __ldg(base4 + v);
       }
 #pragma unroll
       for (int q = 0; q < kArgVecs; ++q) {
-        const int v = v0 + q * kThreads + tid;
-        if (v < nvec) {
-          const T* p = reinterpret_cast<const T*>(&raw[q]);
-#pragma unroll
-          for (int j = 0; j < kPerVec; ++j) {
-            float x;
-            if constexpr (kRawU16) {
-              x = (float)p[j];  // sample<uint16_t> compares the raw integers
-            } else {
-              x = to_f32(p[j]);
-            }
-            if (x > best) {
-              best = x;
-              besti = v * kPerVec + j;
-            }
+        const int v = v0 + q * kArgThreads + tid;
+        if (v < end) {
+          const float x = vec_max<T>(raw[q]);
+          if (x > best) {
+            best = x;
+            bestv = v;
           }
         }
       }
     }
-    for (int i = nvec * kPerVec + tid; i < vocab; i += kThreads) {
-      float x;
-      if constexpr (kRawU16) {
-        x = (float)row[i];
-      } else {
-        x = to_f32(row[i]);
-      }
-      if (x > best) {
-        best = x;
-        besti = i;
-      }
-    }
-    // combine: larger value wins, equal values keep the lower index
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) {
-      const float ov = __shfl_xor_sync(0xffffffffu, best, d);
-      const int oi = __shfl_xor_sync(0xffffffffu, besti, d);
-      if (ov > best || (ov == best && oi < besti)) {
-        best = ov;
-        besti = oi;
-      }
-    }
-    __syncthreads();
-    if (lane == 0) {
-      sv[warp] = best;
-      si[warp] = besti;
-    }
-    __syncthreads();
-    if (tid == 0) {
-      for (int w = 1; w < kWarps; ++w) {
-        if (sv[w] > best || (sv[w] == best && si[w] < besti)) {
-          best = sv[w];
-          besti = si[w];
+    // the row's ragged ends, an element a thread
+    if (rank == 0 && tid < 2 * kPerVec) {
+      const int v = tid < kPerVec ? 0 : nvec - 1;
+      const int i = v * kPerVec + (tid & (kPerVec - 1)) - shift;
+      if ((v < full0 || v >= full1) && i >= 0 && i < vocab) {
+        const float x = arg_value(row[i]);
+        if (x > best || (x == best && x > -INFINITY && v < bestv)) {
+          best = x;
+          bestv = v;
         }
       }
-      // Sequential semantics at the edges: the scan starts from element 0, so if nothing
-      // compares greater than it (all -inf, or element 0 is NaN) the answer is 0. A running
-      // maximum of -inf is only replaced by something greater, so "all -inf" also yields 0.
-      int ans = besti;
-      float first;
-      if constexpr (kRawU16) {
-        first = (float)row[0];
-      } else {
-        first = to_f32(row[0]);
-      }
-      if (first != first) {
-        ans = 0;  // NaN at index 0 is never replaced
-      } else if (besti == 0x7fffffff) {
-        ans = 0;
-      }
-      sv[0] = __int_as_float(ans);
+    }
+    arg_reduce(&best, &bestv);
+    if (lane == 0) {
+      sv[warp] = best;
+      si[warp] = bestv;
     }
     __syncthreads();
-    store_token(out_ids, peers, r, __float_as_int(sv[0]));
+    if (warp == 0) {
+      best = lane < kArgWarps ? sv[lane] : -INFINITY;
+      bestv = lane < kArgWarps ? si[lane] : 0x7fffffff;
+      arg_reduce(&best, &bestv);
+    }
+    if (csize > 1) {
+      cluster_arrive();  // the first block runs before its shared memory is written to
+      cluster_wait();
+      if (tid == 0) {
+        *cluster.map_shared_rank(&cv[rank], 0) = best;
+        *cluster.map_shared_rank(&ci[rank], 0) = bestv;
+      }
+      cluster_arrive();
+      cluster_wait();
+      if (warp == 0 && rank == 0) {
+        best = lane < csize ? cv[lane] : -INFINITY;
+        bestv = lane < csize ? ci[lane] : 0x7fffffff;
+        arg_reduce(&best, &bestv);
+      }
+    }
+    if (rank == 0) {
+      if (warp == 0) {
+        const float first = arg_value(row[0]);
+        int i = 0x7fffffff;
+        if (bestv != 0x7fffffff && lane < kPerVec) {
+          const int j = bestv * kPerVec + lane - shift;
+          if (j >= 0 && j < vocab && arg_value(row[j]) == best) i = j;
+        }
+        i = __reduce_min_sync(0xffffffffu, i);
+        // Sequential semantics at the edges: the scan starts from element 0, so if nothing compares
+        // greater than it (all -inf, or element 0 is NaN) the answer is 0.
+        if (lane == 0) answer = (first != first || i == 0x7fffffff) ? 0 : i;
+      }
+      __syncthreads();
+      store_token(out_ids, peers, r, answer);
+      __syncthreads();
+    }
   }
   peer_arrival_barrier(peers, status);
 }
@@ -843,30 +884,65 @@ cudaError_t launch_sample_rows_ext(
                                    PeerOut{}, scratch, blocks, table, status, settings, pass, stream);
 }
 
+template <typename T, int kArgThreads>
+static cudaError_t launch_argmax_t(
+    const void* logits, int64_t rows, int vocab, int64_t row_stride, int64_t* out_ids, const PeerOut& peers,
+    int csize, int* status, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg = {};
+  if (csize > 8) {
+    static OncePerDevice once;
+    const cudaError_t e = func_attr_once(once, reinterpret_cast<const void*>(argmax_rows_kernel<T, kArgThreads>),
+                                         cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
+  }
+  const int64_t clusters = rows < 1 ? 1 : (rows < (1 << 30) ? rows : (1 << 30));
+  cfg.gridDim = dim3((unsigned)(clusters * csize), 1, 1);
+  cfg.blockDim = dim3(kArgThreads, 1, 1);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)csize;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  programmatic_launch(&attr[1]);
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  return cudaLaunchKernelEx(&cfg, argmax_rows_kernel<T, kArgThreads>, static_cast<const T*>(logits), rows, vocab, row_stride, out_ids,
+                            peers, status);
+}
+
+// Blocks per row: as many as keep two blocks per SM, and leave each thread four loads to have in
+// flight; more of them wait for one another longer than they stream (256 x 128256 bf16: 14.3 us with
+// two blocks per row, 18.6 with eight; one row: 6.6 us with one block, 3.7 with eight). A row per block takes
+// 512 threads while all rows run at once (13.1 us against 14.8 with 256 threads); beyond that smaller
+// blocks make a shorter last wave (400 x 151936 bf16: 22.7 us against 23.8).
+template <typename T>
+static cudaError_t launch_argmax_dtype(
+    const void* logits, int64_t rows, int vocab, int64_t row_stride, int64_t* out_ids, const PeerOut& peers,
+    int sm_count, int* status, cudaStream_t stream) {
+  const int64_t vecs = ((int64_t)vocab * (int64_t)sizeof(T) + 15) / 16;
+  int csize = 1;
+  while (csize < kArgMaxCluster && rows * 2 * csize <= 2 * (int64_t)sm_count && 2 * csize * 4 * 256 <= vecs) csize *= 2;
+  if (csize == 1 && rows <= 2 * (int64_t)sm_count)
+    return launch_argmax_t<T, 512>(logits, rows, vocab, row_stride, out_ids, peers, csize, status, stream);
+  return launch_argmax_t<T, 256>(logits, rows, vocab, row_stride, out_ids, peers, csize, status, stream);
+}
+
 cudaError_t launch_argmax_rows(
     int dtype, const void* logits, int64_t rows, int vocab, int64_t row_stride, int64_t* out_ids,
-    const PeerOut& peers, int blocks, int* status, cudaStream_t stream) {
+    const PeerOut& peers, int sm_count, int* status, cudaStream_t stream) {
   switch (dtype) {
     case kDtypeFloat:
-      argmax_rows_kernel<float, false><<<blocks, kThreads, 0, stream>>>(
-          static_cast<const float*>(logits), rows, vocab, row_stride, out_ids, peers, status);
-      break;
+      return launch_argmax_dtype<float>(logits, rows, vocab, row_stride, out_ids, peers, sm_count, status, stream);
     case kDtypeHalf:
-      argmax_rows_kernel<__half, false><<<blocks, kThreads, 0, stream>>>(
-          static_cast<const __half*>(logits), rows, vocab, row_stride, out_ids, peers, status);
-      break;
+      return launch_argmax_dtype<__half>(logits, rows, vocab, row_stride, out_ids, peers, sm_count, status, stream);
     case kDtypeBFloat16:
-      argmax_rows_kernel<__nv_bfloat16, false><<<blocks, kThreads, 0, stream>>>(
-          static_cast<const __nv_bfloat16*>(logits), rows, vocab, row_stride, out_ids, peers, status);
-      break;
+      return launch_argmax_dtype<__nv_bfloat16>(logits, rows, vocab, row_stride, out_ids, peers, sm_count, status, stream);
     case kDtypeUInt16:
-      argmax_rows_kernel<unsigned short, true><<<blocks, kThreads, 0, stream>>>(
-          static_cast<const unsigned short*>(logits), rows, vocab, row_stride, out_ids, peers, status);
-      break;
+      return launch_argmax_dtype<unsigned short>(logits, rows, vocab, row_stride, out_ids, peers, sm_count, status, stream);
     default:
       return cudaErrorInvalidValue;
   }
-  return cudaGetLastError();
 }
 
 int sample_kernel_max_blocks_per_sm(int dtype) {

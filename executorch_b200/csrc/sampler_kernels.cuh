@@ -122,7 +122,7 @@ cudaError_t launch_fast_rows(
 // temperature == 0: greedy argmax of every row.
 cudaError_t launch_argmax_rows(
     int dtype, const void* logits, int64_t rows, int vocab, int64_t row_stride, int64_t* out_ids,
-    const PeerOut& peers, int blocks, int* status, cudaStream_t stream);
+    const PeerOut& peers, int sm_count, int* status, cudaStream_t stream);
 
 // Value stored into `status` when the arrival barrier of PeerOut gave up waiting for a rank.
 constexpr int kStatusPeerTimeout = 2;

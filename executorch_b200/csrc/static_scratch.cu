@@ -127,9 +127,8 @@ etb200_error_t etb200_sample_rows_static(
   const float inv_t = (temperature != 0.0f) ? 1.0f / temperature : 0.0f;  // sampler.cpp:179
   cudaError_t e;
   if (inv_t == 0.0f) {
-    const int64_t cap = (int64_t)sms * 4;
     e = launch_argmax_rows(dtype, logits_device, rows, vocab_size, row_stride_elems, out_ids_device,
-                           PeerOut{}, (int)(rows < cap ? rows : cap), nullptr, st);
+                           PeerOut{}, sms, nullptr, st);
   } else {
     if (dtype == kDtypeUInt16)
       return fail(ETB200_NOT_SUPPORTED, "UInt16 logits can only be sampled at temperature 0");
