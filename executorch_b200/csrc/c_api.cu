@@ -6,6 +6,7 @@
 
 #include <cstdarg>
 #include <cstdio>
+#include <cstring>
 #include <ctime>
 #include <new>
 
@@ -31,8 +32,10 @@ struct etb200_sampler {
   // staging for the host-buffer entry point
   void* d_stage = nullptr;
   size_t stage_bytes = 0;
-  unsigned long long* d_stage_states = nullptr;
-  int64_t* d_stage_ids = nullptr;
+  // RNG states and ids of a host-buffer call, `stage_rows` of each: pinned memory that the kernels
+  // read and write across the bus (16 bytes per row), which spares three copies per call
+  unsigned long long* h_stage = nullptr;
+  unsigned long long* h_stage_dev = nullptr;
   int64_t stage_rows = 0;
   // the host-buffer entry point copies in slices on its own stream while earlier slices are
   // being sampled on the caller's stream
@@ -343,8 +346,7 @@ etb200_error_t etb200_sampler_destroy(etb200_sampler_t* h) {
   cudaFree(h->d_heads);
   cudaFree(h->fast_scratch);
   cudaFree(h->d_stage);
-  cudaFree(h->d_stage_states);
-  cudaFree(h->d_stage_ids);
+  cudaFreeHost(h->h_stage);
   if (h->copy_stream) cudaStreamDestroy(h->copy_stream);
   for (cudaEvent_t ev : h->slice_ready)
     if (ev) cudaEventDestroy(ev);
@@ -604,22 +606,19 @@ etb200_error_t etb200_sampler_sample_rows_host(
   }
   if (rows > h->stage_rows) {
     ETB_CUDA(cudaDeviceSynchronize());
-    cudaFree(h->d_stage_states);
-    cudaFree(h->d_stage_ids);
-    h->d_stage_states = nullptr;
-    h->d_stage_ids = nullptr;
+    cudaFreeHost(h->h_stage);
+    h->h_stage = nullptr;
     h->stage_rows = 0;
-    cudaError_t e = cudaMalloc(&h->d_stage_states, sizeof(unsigned long long) * (size_t)rows);
-    if (e == cudaSuccess) e = cudaMalloc(&h->d_stage_ids, sizeof(int64_t) * (size_t)rows);
+    cudaError_t e = cudaHostAlloc(&h->h_stage, 2 * sizeof(uint64_t) * (size_t)rows, cudaHostAllocMapped);
+    if (e == cudaSuccess) e = cudaHostGetDevicePointer(&h->h_stage_dev, h->h_stage, 0);
     if (e != cudaSuccess)
-      return fail(ETB200_MEMORY_ALLOCATION_FAILED, "cudaMalloc of staging ids/states failed: %s",
+      return fail(ETB200_MEMORY_ALLOCATION_FAILED, "cudaHostAlloc of staging ids/states failed: %s",
                   cudaGetErrorString(e));
     h->stage_rows = rows;
   }
-  if (!greedy) {
-    ETB_CUDA(cudaMemcpyAsync(h->d_stage_states, rng_states_host, sizeof(uint64_t) * (size_t)rows,
-                             cudaMemcpyHostToDevice, st));
-  }
+  unsigned long long* const states_dev = h->h_stage_dev;
+  int64_t* const ids_dev = reinterpret_cast<int64_t*>(h->h_stage_dev + h->stage_rows);
+  if (!greedy) std::memcpy(h->h_stage, rng_states_host, sizeof(uint64_t) * (size_t)rows);
   // Large batches go in slices of whole rows: slice k+1 crosses PCIe on the handle's copy
   // stream while slice k is sampled on the caller's stream, so that only the last slice's
   // kernel is not hidden behind the copy. Slices stay above 32 rows and 4 MB each.
@@ -633,8 +632,7 @@ etb200_error_t etb200_sampler_sample_rows_host(
   }
   if (slices == 1) {
     ETB_CUDA(cudaMemcpyAsync(h->d_stage, logits_host, bytes, cudaMemcpyHostToDevice, st));
-    err = sample_rows_device(h, h->d_stage, dtype, rows, row_stride_elems, h->d_stage_states,
-                             h->d_stage_ids, st);
+    err = sample_rows_device(h, h->d_stage, dtype, rows, row_stride_elems, states_dev, ids_dev, st);
     if (err != ETB200_OK) return err;
   } else {
     if (!h->copy_stream) {
@@ -657,21 +655,17 @@ etb200_error_t etb200_sampler_sample_rows_host(
       ETB_CUDA(cudaMemcpyAsync(dst + off, src + off, len, cudaMemcpyHostToDevice, h->copy_stream));
       ETB_CUDA(cudaEventRecord(h->slice_ready[k], h->copy_stream));
       ETB_CUDA(cudaStreamWaitEvent(st, h->slice_ready[k], 0));
-      err = sample_rows_device(h, dst + off, dtype, n, row_stride_elems, h->d_stage_states + r0,
-                               h->d_stage_ids + r0, st);
+      err = sample_rows_device(h, dst + off, dtype, n, row_stride_elems, states_dev + r0, ids_dev + r0, st);
       if (err != ETB200_OK) {
         cudaStreamSynchronize(h->copy_stream);
+        cudaStreamSynchronize(st);  // the slices in flight use the staging memory
         return err;
       }
     }
   }
-  ETB_CUDA(cudaMemcpyAsync(out_ids_host, h->d_stage_ids, sizeof(int64_t) * (size_t)rows,
-                           cudaMemcpyDeviceToHost, st));
-  if (!greedy) {
-    ETB_CUDA(cudaMemcpyAsync(rng_states_host, h->d_stage_states, sizeof(uint64_t) * (size_t)rows,
-                             cudaMemcpyDeviceToHost, st));
-  }
   ETB_CUDA(cudaStreamSynchronize(st));
+  std::memcpy(out_ids_host, h->h_stage + h->stage_rows, sizeof(int64_t) * (size_t)rows);
+  if (!greedy) std::memcpy(rng_states_host, h->h_stage, sizeof(uint64_t) * (size_t)rows);
   return ETB200_OK;
 }
 
